@@ -89,8 +89,9 @@ def draw(rng):
                  renorm=rng.random() < 0.8, aux=0.01 if path == "train" else 0.0)
 
 
-def prepare(case, seed):
-    """The layer with its weights, and one batch of rows."""
+def _inputs(case, seed):
+    """Router bias, weights (router, gate, up, down), rows, gradient of the output and the block's gamma; None where the
+    path has none."""
     T, d, dff, E = case["T"], case["d"], case["dff"], case["E"]
     dt, io = DTYPE[case["compute"]], DTYPE[case["io"]]
     g = torch.Generator(device="cuda").manual_seed(seed)
@@ -98,20 +99,31 @@ def prepare(case, seed):
     def rn(*shape, std=1.0, dtype=io):
         return torch.randn(*shape, generator=g, device="cuda").mul_(std).to(dtype)
 
-    layer = MoELayer(d, dff, E, case["k"], bias=case["zipf"], t_max=T, compute_dtype=dt, renormalize=case["renorm"])
     bias = None
     if case["zipf"]:
         rank = torch.randperm(E, generator=g, device="cuda") + 1
         bias = (2.0 * rank.double() ** -1.1).to(dt)
-    layer.setWeights(rn(E, d, std=0.02, dtype=dt), rn(E, dff, d, std=0.02, dtype=dt), rn(E, dff, d, std=0.02, dtype=dt),
-                     rn(E, d, dff, std=0.02, dtype=dt), bias)
-    s = {"case": case, "layer": layer, "x": rn(T, d)}
-    if case["path"].startswith("train"):
+    weights = [rn(E, d, std=0.02, dtype=dt), rn(E, dff, d, std=0.02, dtype=dt), rn(E, dff, d, std=0.02, dtype=dt),
+               rn(E, d, dff, std=0.02, dtype=dt)]
+    x = rn(T, d)
+    dy = rn(T, d) if case["path"].startswith("train") else None
+    gamma = 1.0 + rn(d, std=0.1, dtype=torch.float32) if "block" in case["path"] else None
+    return bias, weights, x, dy, gamma
+
+
+def prepare(case, seed):
+    """The layer with its weights, and one batch of rows."""
+    layer = MoELayer(case["d"], case["dff"], case["E"], case["k"], bias=case["zipf"], t_max=case["T"],
+                     compute_dtype=DTYPE[case["compute"]], renormalize=case["renorm"])
+    bias, weights, x, dy, gamma = _inputs(case, seed)
+    layer.setWeights(*weights, bias)
+    s = {"case": case, "layer": layer, "x": x}
+    if dy is not None:
         layer.set_training(True)
         layer.set_aux_loss(case["aux"])
-        s["dy"] = rn(T, d)
-    if "block" in case["path"]:
-        s["gamma"] = 1.0 + rn(d, std=0.1, dtype=torch.float32)
+        s["dy"] = dy
+    if gamma is not None:
+        s["gamma"] = gamma
     if case["path"] == "host":
         s["x"] = s["x"].cpu().pin_memory()
         s["y"] = torch.empty_like(s["x"]).pin_memory()
@@ -159,3 +171,61 @@ def tolerance(case):
     if case["compute"] == "f32":
         return {"rel": 5e-6, "max": 4e-5}
     return {"rel": 1.7e-2, "max": 0.1} if case["path"].startswith("train") else {"rel": 1.2e-2, "max": 6e-2}
+
+
+def exact(case, seed):
+    """The same outputs in 64 bits.  Picks are taken from the logits of the rows the router sees, which the block form
+    hands over in the layer's element type; nothing else is rounded."""
+    T, d, E, k = (case[n] for n in ("T", "d", "E", "k"))
+    bias, (w_r, w_g, w_u, w_d), x, dy, gamma = _inputs(case, seed)
+    x0 = x.double()
+    xn = x0
+    if gamma is not None:
+        inv = (x0.square().mean(1, keepdim=True) + 1e-5).rsqrt()
+        xn = x0 * inv * gamma.double()
+    rows = xn.to(w_r.dtype).double() if gamma is not None else xn
+    b = bias.double() if bias is not None else 0.0
+    picks = (rows @ w_r.double().T + b).topk(k, dim=1).indices
+    p = (xn @ w_r.double().T + b).softmax(1)
+    pk = p.gather(1, picks)
+    w = pk / pk.sum(1, keepdim=True) if case["renorm"] else pk
+    y = x0.clone() if gamma is not None else torch.zeros_like(x0)
+    if dy is not None:
+        g0 = dy.double()
+        dw, dx = torch.zeros_like(w), torch.zeros_like(x0)
+        keep = torch.float64 if case["compute"] == "f32" else torch.float32  # rounds the large ones once, at the end
+        grads = {n: torch.zeros(m.shape, dtype=keep, device="cuda") for n, m in
+                 (("d_gate", w_g), ("d_up", w_u), ("d_down", w_d))}
+    for e in range(E):
+        t, j = (picks == e).nonzero(as_tuple=True)
+        if not len(t):
+            continue
+        wg, wu, wd, xe, we = w_g[e].double(), w_u[e].double(), w_d[e].double(), xn[t], w[t, j].unsqueeze(1)
+        g, u = xe @ wg.T, xe @ wu.T
+        sg = g.sigmoid()
+        h = g * sg * u
+        ye = h @ wd.T
+        y.index_add_(0, t, we * ye)
+        if dy is not None:
+            dye = g0[t]
+            dw[t, j] = (dye * ye).sum(1)
+            dye = we * dye
+            dh = dye @ wd
+            dg, du = dh * u * sg * (1.0 + g * (1.0 - sg)), dh * g * sg
+            grads["d_gate"][e], grads["d_up"][e], grads["d_down"][e] = dg.T @ xe, du.T @ xe, dye.T @ h
+            dx.index_add_(0, t, dg @ wg + du @ wu)
+    if dy is None:
+        return y.cpu() if case["path"] == "host" else y
+    dpk = (dw - (dw * w).sum(1, keepdim=True)) / pk.sum(1, keepdim=True) if case["renorm"] else dw
+    load = torch.bincount(picks.flatten(), minlength=E).double() / (T * k)
+    dp = (case["aux"] * E / T * load).expand(T, E).scatter_add(1, picks, dpk)
+    dl = p * (dp - (p * dp).sum(1, keepdim=True))
+    grads["d_router"], grads["d_bias"] = dl.T @ xn, dl.sum(0)
+    dx += dl @ w_r.double()
+    grads = {n: grads[n] for n in ("d_router", "d_bias", "d_gate", "d_up", "d_down")}
+    if gamma is None:
+        return dict(grads, y=y, dx=dx)
+    dgamma = (x0 * inv * dx).sum(0)
+    dn = dx * gamma.double()
+    dx = g0 + inv * (dn - x0 * inv.square() * (dn * x0).mean(1, keepdim=True))
+    return dict(grads, y=y, dx=dx, dgamma=dgamma)
