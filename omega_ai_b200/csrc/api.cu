@@ -117,7 +117,7 @@ int omoe_destroy(omoe_handle *h) {
     if (!h) return OMOE_OK;
     ep_destroy(h);
     bw_destroy(h);
-    void *ptrs[] = {h->w_router, h->w_router_bf16, h->router_bias, h->w_gate, h->w_up, h->w_down, h->logits, h->topk_idx,
+    void *ptrs[] = {h->w_router, h->w_router_bf16, h->router_bias, h->w_gate, h->w_down, h->logits, h->topk_idx,
                     h->topk_w, h->block_counts, h->block_base, h->counts, h->offsets, h->poffsets, h->tile_expert, h->pos, h->lrank,
                     h->perm_out, h->dev_err, h->xp, h->hbuf, h->yp, h->xn, h->x_stage[0], h->y_stage[0], h->x_stage[1], h->y_stage[1], h->d_row_table,
                     h->d_out_table, h->ticket, h->ticket2, h->ticket3, h->dst_base != h->poffsets ? h->dst_base : nullptr};
@@ -205,8 +205,8 @@ int omoe_create(const omoe_config *cfg, omoe_handle **out) {
     if (c.has_router_bias) ALLOC(router_bias, E);
     {
         struct { void **p; size_t bytes; } bufs[] = {
-            {&h->w_gate, (size_t)h->e_local * dff * d * cs}, {&h->w_up, (size_t)h->e_local * dff * d * cs},
-            {&h->w_down, (size_t)h->e_local * dff * d * cs}, {&h->xp, (size_t)h->rows_cap * d * cs},
+            {&h->w_gate, (size_t)h->e_local * dff * d * cs * 2}, {&h->w_down, (size_t)h->e_local * dff * d * cs},
+            {&h->xp, (size_t)h->rows_cap * d * cs},
             {&h->hbuf, (size_t)h->rows_cap * dff * cs},      {&h->yp, (size_t)h->rows_cap * d * cs},
             {&h->x_stage[0], (size_t)tm * d * 4},            {&h->y_stage[0], (size_t)tm * d * 4},
             {&h->x_stage[1], (size_t)tm * d * 4},            {&h->y_stage[1], (size_t)tm * d * 4},
@@ -223,6 +223,7 @@ int omoe_create(const omoe_config *cfg, omoe_handle **out) {
             }
         }
     }
+    h->w_up = static_cast<char *>(h->w_gate) + (size_t)h->e_local * dff * d * cs;
     ALLOC(logits, tm * E);
     ALLOC(topk_idx, tm * k);
     ALLOC(topk_w, tm * k);

@@ -14,7 +14,7 @@ if [ "$1" = "check" ]; then
     OMOE_NVCC_EXTRA="$OMOE_NVCC_EXTRA -DOMOE_BOUNDS_CHECK"
 fi
 FLAGS="-gencode arch=compute_100a,code=sm_100a -O3 -lineinfo -std=c++17 -Xcompiler -fPIC -Xcompiler -fvisibility=hidden ${OMOE_NVCC_EXTRA}"
-SRCS="api.cu rmsnorm.cu router.cu route_small.cu permute.cu combine.cu experts_f32.cu experts_sm100.cu experts_sm100_splitk.cu experts_sm100_wgrad.cu backward.cu experts_decode.cu ep.cu check.cu"
+SRCS="api.cu rmsnorm.cu router.cu route_small.cu permute.cu combine.cu experts_f32.cu experts_sm100.cu experts_sm100_pair.cu experts_sm100_splitk.cu experts_sm100_wgrad.cu backward.cu experts_decode.cu ep.cu check.cu"
 mkdir -p "$OBJDIR"
 # a changed flag set rebuilds everything
 echo "$FLAGS" > "$OBJDIR/flags.new"

@@ -9,6 +9,7 @@
 #include <stdio.h>
 
 #include "../../include/omoe.h"
+#include "pair.cuh"
 #include "pdl.cuh"
 #include "vec8.cuh"
 
@@ -56,6 +57,7 @@ struct TensorMaps {
     CUtensorMap b_down;  // [E_local*d, dff]
     CUtensorMap c_y;     // expert outputs yp [rows_cap, d] (store target)
     CUtensorMap a_x32, a_h32;  // xp and h with a 32-row box (tiles with few tokens, split-K kernels)
+    PairMaps up, down;         // the products on pairs of SMs (experts_sm100_pair.cu)
 };
 
 }  // namespace omoe
@@ -75,7 +77,7 @@ struct omoe_handle {
     float *w_router;      // [E, d] fp32
     float *router_bias;   // [E] fp32 or null
     __nv_bfloat16 *w_router_bf16;  // [E, d] copy, only while the router weights were given as bf16 (exact)
-    void *w_gate, *w_up;  // [E_local, dff, d] compute dtype
+    void *w_gate, *w_up;  // [E_local, dff, d] compute dtype, one allocation: w_up follows w_gate
     void *w_down;         // [E_local, d, dff]
 
     // routing workspace (device)

@@ -403,6 +403,20 @@ bool build_tensor_maps(omoe_handle *h) {
               encode_map(fn, &h->maps.b_up, h->w_up, El * dff, d) &&
               encode_map(fn, &h->maps.b_down, h->w_down, El * d, dff) && encode_map(fn, &h->maps.c_y, h->yp, rows, d) &&
               encode_map(fn, &h->maps.a_x32, h->xp, rows, d, 32) && encode_map(fn, &h->maps.a_h32, h->hbuf, rows, dff, 32);
+    {
+        // up/gate: 8 gate rows, then 8 up rows, then the next 8 gate rows ...: w_up follows w_gate in memory
+        const uint64_t dims[4] = {d, 8, 2, El * dff / 8}, strides[3] = {d, El * dff * d, 8 * d};
+        const uint32_t box[4] = {BLOCK_K, 8, 2, 8};
+        PairMaps &u = h->maps.up, &w = h->maps.down;
+        ok = ok && encode_map_nd(&u.a0, h->w_gate, 4, dims, strides, box) &&
+             encode_map(fn, &u.o0, h->hbuf, rows, dff, 32);
+        u.b0 = h->maps.a_x;
+        u.b0_32 = h->maps.a_x32;
+        w.a0 = h->maps.b_down;
+        w.b0 = h->maps.a_h;
+        w.b0_32 = h->maps.a_h32;
+        ok = ok && encode_map(fn, &w.o0, h->yp, rows, d, 32);
+    }
     if (!ok) snprintf(h->err, sizeof(h->err), "cuTensorMapEncodeTiled failed (d=%d, d_ff=%d)", (int)d, (int)dff);
     h->maps_ready = ok;
     return ok;
@@ -422,6 +436,23 @@ cudaError_t set_smem_attrs() {
     return cudaSuccess;
 }
 }  // namespace
+
+bool encode_map_nd(CUtensorMap *m, void *ptr, int rank, const uint64_t *dims, const uint64_t *strides, const uint32_t *box,
+                   bool f32) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (!fn || rank < 2 || rank > 5) return false;
+    cuuint64_t dm[5], st[4];
+    cuuint32_t bx[5], estr[5];
+    for (int i = 0; i < rank; i++) {
+        dm[i] = dims[i];
+        bx[i] = box[i];
+        estr[i] = 1;
+        if (i > 0) st[i - 1] = strides[i - 1] * (f32 ? 4 : 2);
+    }
+    return fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, ptr, dm, st, bx,
+              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 bool encode_map_bf16(CUtensorMap *m, void *ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
     EncodeTiledFn fn = get_encode_fn();
@@ -483,6 +514,8 @@ cudaError_t launch_experts_bf16(omoe_handle *h, cudaStream_t s, int *n, cudaEven
     cudaError_t e;
     if (s_up > 0) {
         e = launch_up_gate_splitk(h, s, s_up, gate ? &g_up : nullptr);
+    } else if (gate == nullptr) {
+        e = launch_pair(h, s, h->pdl, PairKind::kUpGate, h->maps.up, dff, d, 32);
     } else {
         e = launch_ex(grouped_gemm_kernel<true>, grid, block, kSmemBytes, s, h->pdl, h->maps.a_x, h->maps.b_gate,
                       h->maps.b_up, h->maps.a_h, dff, d, h->ex_tile_expert, h->ex_poffsets, h->e_local, band_up,
@@ -493,6 +526,11 @@ cudaError_t launch_experts_bf16(omoe_handle *h, cudaStream_t s, int *n, cudaEven
     if (mid) cudaEventRecord(mid, s);
     if (s_dn > 0) {
         e = launch_down_splitk(h, s, s_dn, gate ? &g_dn : nullptr);
+        if (e == cudaSuccess) (*n)++;
+        return e;
+    }
+    if (gate == nullptr) {
+        e = launch_pair(h, s, h->pdl, PairKind::kPlain, h->maps.down, d, dff, 32);
         if (e == cudaSuccess) (*n)++;
         return e;
     }
