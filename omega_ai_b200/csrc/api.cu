@@ -356,7 +356,6 @@ int omoe_set_weights(omoe_handle *h, const void *w_router, const void *router_bi
         }
     }
     h->weights_set = true;
-    bw_weights_changed(h);
     return OMOE_OK;
 }
 

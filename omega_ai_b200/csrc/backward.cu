@@ -13,15 +13,15 @@
 // dx[t] = sum of the picks' dxp rows in pick order plus the router's term, added last.
 //
 // A forward in training mode keeps what this needs: the pre-activation rows g and u (one buffer
-// [rows, 2*d_ff], g in the left half), h, yp and the routing.  The fused SiLU epilogue of the inference
-// forward cannot keep g and u, so the training forward runs the up/gate products as two plain products
-// plus one element-wise pass.
+// [rows, 2*d_ff], g in the left half), h, yp and the routing.
 //
-// bf16 layers: every product runs on the tcgen05 kernels.  The two input-gradient products are the
-// forward's persistent kernel on transposed copies of the weights (W_down^T, and [W_gate^T | W_up^T] so
-// that dxp = [dg | du] * [W_gate ; W_up] is ONE product over K = 2*d_ff); the weight-gradient products
-// (experts_sm100_wgrad.cu) reduce over an expert's rows, so their operands are the transposed
-// activations, written by a pass that also zero-fills each expert's padding rows.
+// bf16 layers: every product runs on pairs of SMs (experts_sm100_pair.cu, experts_sm100_wgrad.cu).  The training
+// forward's up/gate product stores g and u beside h from one accumulator.  The two input-gradient products read the
+// forward's weights as they lie, as MN-major operands (dxp = dg * W_gate + du * W_up is ONE product with two sources), so
+// there are no transposed copies to refresh when the weights change: on the Mixtral-shaped layer those were 2.8 GB of
+// memory and three passes over the weights after every omoe_set_weights.  The weight-gradient products reduce over an
+// expert's rows and read the activations in place; padding rows are zeroed in xp and dyp, hence zero in everything
+// derived from them.
 // fp32 layers: a plain tiled FMA kernel with strided operands (sized for parity runs, not for speed).
 #include <stdlib.h>
 #include <string.h>
@@ -38,7 +38,6 @@ namespace omoe {
 struct BwState {
     bool training;
     bool fwd_valid;   // the last forward ran in training mode and its saved rows are intact
-    bool wt_valid;    // transposed weight copies match the current weights
     int fwd_T;
     float aux_coef;   // weight of the auxiliary load-balancing loss in the objective (0: none)
     float *aux_ps;    // [E] column sums of the router probabilities (omoe_get_aux_loss)
@@ -55,19 +54,11 @@ struct BwState {
     float *dl;        // [t_max, E] gradient of the logits
     float *dwr_part;  // [slices][E][d] partial sums of d W_router
     int dwr_slices;
-    // bf16 layers only
-    void *wdT;        // [El, dff, d]     W_down^T
-    void *wguT;       // [El, d, 2*dff]   [W_gate^T | W_up^T]
-    void *xpT, *hT, *dypT, *dguT;  // [cols, rows_cap] transposed activations
     // gradients (fp32)
     float *d_router, *d_bias, *d_gate, *d_up, *d_down;
     // tensor maps of the bf16 products
-    CUtensorMap m_g_out, m_u_out;          // halves of gu as store targets
-    CUtensorMap m_dyp_a, m_wdT_b, m_dh_c;  // dh = dyp * W_down
-    CUtensorMap m_dgu_a, m_wguT_b, m_dxp_c;  // dxp = [dg|du] * [Wg;Wu]
-    CUtensorMap m_dypT, m_hT, m_dguT, m_xpT;  // weight-gradient operands, transposed copies (older path)
-    CUtensorMap m_dyp_r, m_h_r, m_dgu_r, m_xp_r;  // weight-gradient operands read in place (64-row boxes)
-    bool wgrad_transposed;  // OMOE_WGRAD_TRANSPOSED=1: use the transposed copies
+    PairMaps up, dh_maps, dxp_maps;  // up/gate keeping g and u; dyp * W_down; dg * W_gate + du * W_up
+    WgradMaps w_down, w_gu;
 };
 
 namespace {
@@ -353,52 +344,6 @@ zero_pad_rows_kernel(T *__restrict__ buf, int ld, const int32_t *__restrict__ po
         base[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// ---- transposes (bf16 layers) ---------------------------------------------------------------------
-// dst[c, r] = src[r, c] for the rows in use, r < *rows_in_use (a multiple of 128); rows of an expert's
-// segment beyond its count are written as zeros, so a reduction over the padded segment adds nothing.
-// src [rows, C] with leading dimension ld_src; dst [C, ld_dst].  64 x 64 tiles through shared memory.
-__global__ void __launch_bounds__(256)
-transpose_rows_kernel(const __nv_bfloat16 *__restrict__ src, int ld_src, __nv_bfloat16 *__restrict__ dst, int ld_dst,
-                      int C, const int32_t *__restrict__ rows_in_use, const int32_t *__restrict__ tile_expert,
-                      const int32_t *__restrict__ poffsets, const int32_t *__restrict__ counts) {
-    __shared__ __nv_bfloat16 tile[64][66];
-    const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
-    if (r0 >= *rows_in_use) return;
-    const int e = tile_expert[r0 / kRowAlign];
-    const int valid_end = poffsets[e] + counts[e];  // rows of this segment at or beyond it are padding
-    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;  // 64 x 4
-    for (int i = ty; i < 64; i += 4) {
-        const int r = r0 + i, c = c0 + tx;
-        tile[i][tx] = (r < valid_end && c < C) ? src[(size_t)r * ld_src + c] : __float2bfloat16_rn(0.f);
-    }
-    __syncthreads();
-    for (int i = ty; i < 64; i += 4) {
-        const int c = c0 + i, r = r0 + tx;
-        if (c < C) dst[(size_t)c * ld_dst + r] = tile[tx][i];
-    }
-}
-
-// Batched plain transpose: for each batch b, dst_b[c, r] = src_b[r, c]; src_b = src + b*R*C ([R, C]);
-// dst_b = dst + b*dst_batch + dst_col0, leading dimension ld_dst.
-__global__ void __launch_bounds__(256)
-transpose_batched_kernel(const __nv_bfloat16 *__restrict__ src, __nv_bfloat16 *__restrict__ dst, int R, int C,
-                         int ld_dst, size_t dst_batch, int dst_col0) {
-    __shared__ __nv_bfloat16 tile[64][66];
-    const __nv_bfloat16 *s = src + (size_t)blockIdx.z * R * C;
-    __nv_bfloat16 *o = dst + (size_t)blockIdx.z * dst_batch + dst_col0;
-    const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
-    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-    for (int i = ty; i < 64; i += 4) {
-        const int r = r0 + i, c = c0 + tx;
-        if (r < R && c < C) tile[i][tx] = s[(size_t)r * C + c];
-    }
-    __syncthreads();
-    for (int i = ty; i < 64; i += 4) {
-        const int c = c0 + i, r = r0 + tx;
-        if (c < C && r < R) o[(size_t)c * ld_dst + r] = tile[tx][i];
-    }
-}
-
 // ---- fp32 products (parity-sized) -----------------------------------------------------------------
 // Rows grouped by expert: C[r, n] (+)= sum_k A[r, k] * B_e(k, n) for the rows in use, where the expert of
 // a row comes from its 128-row tile and B_e(k, n) = B[e*sbe + k*sbk + n*sbn].  64 x 64 tiles, 4 x 4 per thread.
@@ -502,8 +447,8 @@ cudaError_t forward_experts_t(omoe_handle *h, BwState *b, cudaStream_t s, int *n
     BW_TRY(cudaGetLastError());
     (*n)++;
     if constexpr (sizeof(CT) == 2) {
-        BW_TRY(launch_grouped_plain(h, s, h->maps.a_x, h->maps.b_gate, b->m_g_out, dff, d));
-        BW_TRY(launch_grouped_plain(h, s, h->maps.a_x, h->maps.b_up, b->m_u_out, dff, d));
+        BW_TRY(launch_pair(h, s, false, PairKind::kUpGateKeep, b->up, dff, d, 64));
+        (*n)++;
     } else {
         dim3 grid((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(dff, 64));
         const float *xp = static_cast<const float *>(h->xp);
@@ -514,15 +459,13 @@ cudaError_t forward_experts_t(omoe_handle *h, BwState *b, cudaStream_t s, int *n
         sgemm_rows_kernel<<<grid, 256, 0, s>>>(xp, d, static_cast<const float *>(h->w_up), (size_t)dff * d, 1, d,
                                                reinterpret_cast<float *>(gu) + dff, 2 * dff, dff, d, rows_in_use,
                                                h->ex_tile_expert, 0);
+        swiglu_fwd_kernel<CT><<<grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count), 256, 0, s>>>(
+            gu, static_cast<CT *>(h->hbuf), rows_in_use, dff);
         BW_TRY(cudaGetLastError());
+        *n += 3;
     }
-    *n += 2;
-    swiglu_fwd_kernel<CT><<<grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count), 256, 0, s>>>(
-        gu, static_cast<CT *>(h->hbuf), rows_in_use, dff);
-    BW_TRY(cudaGetLastError());
-    (*n)++;
     if constexpr (sizeof(CT) == 2) {
-        BW_TRY(launch_grouped_plain(h, s, h->maps.a_h, h->maps.b_down, h->maps.c_y, d, dff));
+        BW_TRY(launch_pair(h, s, false, PairKind::kPlain, h->maps.down, d, dff, 32));
     } else {
         dim3 grid((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(d, 64));
         // yp[r, c] = sum_f h[r, f] * Wd[e][c][f]
@@ -533,24 +476,6 @@ cudaError_t forward_experts_t(omoe_handle *h, BwState *b, cudaStream_t s, int *n
         BW_TRY(cudaGetLastError());
     }
     (*n)++;
-    return cudaSuccess;
-}
-
-cudaError_t transpose_weights(omoe_handle *h, BwState *b, cudaStream_t s, int *n) {
-    const int d = h->cfg.d_model, dff = h->cfg.d_ff, El = h->e_local;
-    auto *wg = static_cast<const __nv_bfloat16 *>(h->w_gate), *wu = static_cast<const __nv_bfloat16 *>(h->w_up);
-    auto *wd = static_cast<const __nv_bfloat16 *>(h->w_down);
-    // W_down [El][d][dff] -> wdT [El][dff][d]
-    transpose_batched_kernel<<<dim3(ceil_div(d, 64), ceil_div(dff, 64), El), 256, 0, s>>>(
-        wd, static_cast<__nv_bfloat16 *>(b->wdT), d, dff, d, (size_t)dff * d, 0);
-    // W_gate, W_up [El][dff][d] -> wguT [El][d][2*dff] (gate in columns [0, dff), up in [dff, 2*dff))
-    transpose_batched_kernel<<<dim3(ceil_div(dff, 64), ceil_div(d, 64), El), 256, 0, s>>>(
-        wg, static_cast<__nv_bfloat16 *>(b->wguT), dff, d, 2 * dff, (size_t)d * 2 * dff, 0);
-    transpose_batched_kernel<<<dim3(ceil_div(dff, 64), ceil_div(d, 64), El), 256, 0, s>>>(
-        wu, static_cast<__nv_bfloat16 *>(b->wguT), dff, d, 2 * dff, (size_t)d * 2 * dff, dff);
-    BW_TRY(cudaGetLastError());
-    *n += 3;
-    b->wt_valid = true;
     return cudaSuccess;
 }
 
@@ -586,43 +511,23 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
     (*n)++;
     const int ew_grid = grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count);
     if constexpr (sizeof(CT) == 2) {
-        if (!b->wt_valid) BW_TRY(transpose_weights(h, b, s, n));
-        // dh = dyp * W_down      (rows x d) * (d x dff): the forward's kernel on W_down^T
-        BW_TRY(launch_grouped_plain(h, s, b->m_dyp_a, b->m_wdT_b, b->m_dh_c, dff, d));
+        // dh = dyp * W_down; rows up to a multiple of 64, because the weight gradients reduce over blocks of 64 rows
+        BW_TRY(launch_pair(h, s, false, PairKind::kPlainMN, b->dh_maps, dff, d, 64));
         (*n)++;
         swiglu_bwd_kernel<CT><<<ew_grid, 256, 0, s>>>(static_cast<const CT *>(b->dh), static_cast<const CT *>(b->gu),
                                                       static_cast<CT *>(b->dgu), rows_in_use, dff);
         BW_TRY(cudaGetLastError());
         (*n)++;
-        // dxp = [dg | du] * [W_gate ; W_up]: one product over K = 2*dff
-        BW_TRY(launch_grouped_plain(h, s, b->m_dgu_a, b->m_wguT_b, b->m_dxp_c, d, 2 * dff));
+        BW_TRY(launch_pair(h, s, false, PairKind::kPlainMN2, b->dxp_maps, d, dff, 32));
         (*n)++;
         if (ep) {
             // the input-gradient rows are complete: the token ranks may fetch them while the weight gradients run
             BW_TRY(ep_signal_out(h, s));
             (*n)++;
         }
-        // d W_down[e] [d, dff] = dyp_e^T * h_e;  [d W_gate ; d W_up][e] [2*dff, d] = [dg | du]_e^T * xp_e
-        if (!b->wgrad_transposed) {
-            // operands read in place as MN-major tiles; dyp's padding rows are zero, hence dh's and [dg|du]'s
-            BW_TRY(launch_wgrad_bf16_rows(h, s, b->m_dyp_r, b->m_h_r, d, dff, d, b->d_down, b->d_down));
-            BW_TRY(launch_wgrad_bf16_rows(h, s, b->m_dgu_r, b->m_xp_r, 2 * dff, d, dff, b->d_gate, b->d_up));
-        } else {
-            // transposed copies with each expert's padding rows zero-filled, then K-major operands
-            auto tr = [&](const void *src, int ld, void *dst, int C) {
-                transpose_rows_kernel<<<dim3((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(C, 64)), 256, 0, s>>>(
-                    static_cast<const __nv_bfloat16 *>(src), ld, static_cast<__nv_bfloat16 *>(dst), (int)h->rows_cap, C,
-                    rows_in_use, h->ex_tile_expert, h->ex_poffsets, h->ex_counts);
-                (*n)++;
-            };
-            tr(b->dyp, d, b->dypT, d);
-            tr(h->hbuf, dff, b->hT, dff);
-            tr(b->dgu, 2 * dff, b->dguT, 2 * dff);
-            tr(h->xp, d, b->xpT, d);
-            BW_TRY(cudaGetLastError());
-            BW_TRY(launch_wgrad_bf16(h, s, b->m_dypT, b->m_hT, d, dff, d, b->d_down, b->d_down));
-            BW_TRY(launch_wgrad_bf16(h, s, b->m_dguT, b->m_xpT, 2 * dff, d, dff, b->d_gate, b->d_up));
-        }
+        // d W_down[e] [d, dff] = dyp_e^T * h_e;  d W_gate[e], d W_up[e] [dff, d] = dg_e^T * xp_e, du_e^T * xp_e
+        BW_TRY(launch_wgrad(h, s, b->w_down, 1, d, dff));
+        BW_TRY(launch_wgrad(h, s, b->w_gu, 2, dff, d));
         *n += 2;
     } else {
         const float *dyp = static_cast<const float *>(b->dyp);
@@ -687,8 +592,7 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
 
 void free_state(BwState *b) {
     if (!b->own_grad_rows) b->dyp = b->dxp = nullptr, b->dyp_table = b->dxp_table = nullptr;
-    void *ptrs[] = {b->dyp_table, b->dxp_table, b->gu, b->dyp, b->dh, b->dgu, b->dxp, b->dgw, b->dl, b->dwr_part, b->wdT, b->wguT, b->xpT, b->hT,
-                    b->dypT, b->dguT, b->d_router, b->d_bias, b->d_gate, b->d_up, b->d_down, b->aux_ps, b->dxn, b->inv_rms};
+    void *ptrs[] = {b->dyp_table, b->dxp_table, b->gu, b->dyp, b->dh, b->dgu, b->dxp, b->dgw, b->dl, b->dwr_part, b->d_router, b->d_bias, b->d_gate, b->d_up, b->d_down, b->aux_ps, b->dxn, b->inv_rms};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete b;
@@ -732,17 +636,6 @@ int bw_set_training(omoe_handle *h, int on) {
             cudaMemcpy(b->dxp_table, &b->dxp, sizeof(void *), cudaMemcpyHostToDevice);
         }
     }
-    const char *wt = getenv("OMOE_WGRAD_TRANSPOSED");
-    b->wgrad_transposed = wt && atoi(wt) != 0;
-    if (ok && cs == 2) {
-        struct { void **p; size_t bytes; } tb[] = {{&b->wdT, El * dff * d * 2}, {&b->wguT, El * d * 2 * dff * 2}};
-        for (auto &x : tb) ok = ok && cudaMalloc(x.p, x.bytes) == cudaSuccess;
-    }
-    if (ok && cs == 2 && b->wgrad_transposed) {
-        struct { void **p; size_t bytes; } tb[] = {{&b->xpT, d * rows * 2}, {&b->hT, dff * rows * 2},
-                                                   {&b->dypT, d * rows * 2}, {&b->dguT, 2 * dff * rows * 2}};
-        for (auto &x : tb) ok = ok && cudaMalloc(x.p, x.bytes) == cudaSuccess;
-    }
     if (!ok) {
         cudaGetLastError();
         free_state(b);
@@ -754,24 +647,38 @@ int bw_set_training(omoe_handle *h, int on) {
     if (b->own_grad_rows) cudaMemset(b->dyp, 0, rows * d * cs);
     cudaMemset(b->dgu, 0, rows * 2 * dff * cs);
     if (cs == 2) {
-        // columns of the transposed buffers beyond the rows in use are never read
-        bool m = encode_map_bf16(&b->m_g_out, b->gu, rows, dff, 2 * dff, 128) &&
-                 encode_map_bf16(&b->m_u_out, static_cast<__nv_bfloat16 *>(b->gu) + dff, rows, dff, 2 * dff, 128) &&
-                 encode_map_bf16(&b->m_dyp_a, b->dyp, rows, d, d, 128) &&
-                 encode_map_bf16(&b->m_wdT_b, b->wdT, El * dff, d, d, 128) &&
-                 encode_map_bf16(&b->m_dh_c, b->dh, rows, dff, dff, 128) &&
-                 encode_map_bf16(&b->m_dgu_a, b->dgu, rows, 2 * dff, 2 * dff, 128) &&
-                 encode_map_bf16(&b->m_wguT_b, b->wguT, El * d, 2 * dff, 2 * dff, 128) &&
-                 encode_map_bf16(&b->m_dxp_c, b->dxp, rows, d, d, 128) &&
-                 encode_map_bf16(&b->m_dyp_r, b->dyp, rows, d, d, 64) &&
-                 encode_map_bf16(&b->m_h_r, h->hbuf, rows, dff, dff, 64) &&
-                 encode_map_bf16(&b->m_dgu_r, b->dgu, rows, 2 * dff, 2 * dff, 64) &&
-                 encode_map_bf16(&b->m_xp_r, h->xp, rows, d, d, 64);
-        if (m && b->wgrad_transposed)
-            m = encode_map_bf16(&b->m_dypT, b->dypT, d, rows, rows, 128) &&
-                encode_map_bf16(&b->m_hT, b->hT, dff, rows, rows, 128) &&
-                encode_map_bf16(&b->m_dguT, b->dguT, 2 * dff, rows, rows, 128) &&
-                encode_map_bf16(&b->m_xpT, b->xpT, d, rows, rows, 128);
+        typedef __nv_bfloat16 bf;
+        bf *gu = static_cast<bf *>(b->gu), *dgu = static_cast<bf *>(b->dgu);
+        // weights as [expert][reduction][output feature]: the boxes end with the expert's matrix
+        auto weights = [&](CUtensorMap *mp, void *w, uint64_t red, uint64_t out) {
+            const uint64_t dims[3] = {out, red, El}, strides[2] = {out, out * red};
+            const uint32_t box[3] = {64, 64, 1};
+            return encode_map_nd(mp, w, 3, dims, strides, box);
+        };
+        auto grads = [&](CUtensorMap *mp, float *g, uint64_t M, uint64_t N) {
+            const uint64_t dims[3] = {N, M, El}, strides[2] = {N, N * M};
+            const uint32_t box[3] = {32, 32, 1};
+            return encode_map_nd(mp, g, 3, dims, strides, box, true);
+        };
+        b->up = h->maps.up;
+        bool m = encode_map_bf16(&b->up.o1, gu, rows, dff, 2 * dff, 32) &&
+                 encode_map_bf16(&b->up.o2, gu + dff, rows, dff, 2 * dff, 32) &&
+                 weights(&b->dh_maps.a0, h->w_down, d, dff) &&
+                 encode_map_bf16(&b->dh_maps.b0, b->dyp, rows, d, d, 128) &&
+                 encode_map_bf16(&b->dh_maps.b0_32, b->dyp, rows, d, d, 32) &&
+                 encode_map_bf16(&b->dh_maps.o0, b->dh, rows, dff, dff, 32) &&
+                 weights(&b->dxp_maps.a0, h->w_gate, dff, d) && weights(&b->dxp_maps.a1, h->w_up, dff, d) &&
+                 encode_map_bf16(&b->dxp_maps.b0, dgu, rows, dff, 2 * dff, 128) &&
+                 encode_map_bf16(&b->dxp_maps.b0_32, dgu, rows, dff, 2 * dff, 32) &&
+                 encode_map_bf16(&b->dxp_maps.b1, dgu + dff, rows, dff, 2 * dff, 128) &&
+                 encode_map_bf16(&b->dxp_maps.b1_32, dgu + dff, rows, dff, 2 * dff, 32) &&
+                 encode_map_bf16(&b->dxp_maps.o0, b->dxp, rows, d, d, 32) &&
+                 encode_map_bf16(&b->w_down.a0, b->dyp, rows, d, d, 64) &&
+                 encode_map_bf16(&b->w_down.b, h->hbuf, rows, dff, dff, 64) && grads(&b->w_down.o0, b->d_down, d, dff) &&
+                 encode_map_bf16(&b->w_gu.a0, dgu, rows, dff, 2 * dff, 64) &&
+                 encode_map_bf16(&b->w_gu.a1, dgu + dff, rows, dff, 2 * dff, 64) &&
+                 encode_map_bf16(&b->w_gu.b, h->xp, rows, d, d, 64) && grads(&b->w_gu.o0, b->d_gate, dff, d) &&
+                 grads(&b->w_gu.o1, b->d_up, dff, d);
         if (!m) {
             free_state(b);
             snprintf(h->err, sizeof(h->err), "omoe_set_training: cuTensorMapEncodeTiled failed");
@@ -788,10 +695,6 @@ int bw_set_training(omoe_handle *h, int on) {
 }
 
 bool bw_training(const omoe_handle *h) { return h->bw && static_cast<BwState *>(h->bw)->training; }
-
-void bw_weights_changed(omoe_handle *h) {
-    if (h->bw) static_cast<BwState *>(h->bw)->wt_valid = false;
-}
 
 void bw_forward_invalidate(omoe_handle *h) {
     if (h->bw) static_cast<BwState *>(h->bw)->fwd_valid = false;

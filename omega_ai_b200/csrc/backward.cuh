@@ -7,7 +7,6 @@ namespace omoe {
 
 int bw_set_training(omoe_handle *h, int on);
 bool bw_training(const omoe_handle *h);
-void bw_weights_changed(omoe_handle *h);
 void bw_forward_invalidate(omoe_handle *h);
 // A training-mode forward of no rows on one GPU launches nothing and still counts as the forward a backward follows.
 void bw_forward_empty(omoe_handle *h);
@@ -26,19 +25,12 @@ void bw_destroy(omoe_handle *h);
 
 // 2-D bf16 tensor map: [rows, cols] with `ld` elements between rows, box box_rows x 64 columns, 128-byte swizzle.
 bool encode_map_bf16(CUtensorMap *m, void *ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows);
-// out[r, 0..n_out) = a[r, 0..K) * B_e^T for the rows in use, B_e = rows [e*n_out, (e+1)*n_out) of b ([.., K]):
-// the persistent tcgen05 kernel of the forward's down product with other operands (experts_sm100.cu).
-cudaError_t launch_grouped_plain(omoe_handle *h, cudaStream_t s, const CUtensorMap &a, const CUtensorMap &b,
-                                 const CUtensorMap &c, int n_out, int K);
-// Per local expert e: C_e [M, N] (fp32) = AT[:, seg_e] * BT[:, seg_e]^T, seg_e = the expert's (padded, zero-filled)
-// rows; at [M, rows_cap], bt [N, rows_cap] bf16.  Row m of C_e goes to out0[e][m][:] when m < split, else to
-// out1[e][m - split][:].  (experts_sm100_wgrad.cu)
-cudaError_t launch_wgrad_bf16(omoe_handle *h, cudaStream_t s, const CUtensorMap &at, const CUtensorMap &bt, int M,
-                              int N, int split, float *out0, float *out1);
-
-// The same product straight from the row-major activations a [rows_cap, M], b [rows_cap, N] (tensor maps with a
-// 64-row box): MN-major tensor-core operands, no transposed copies.  Padding rows of a must be zero, of b finite.
-cudaError_t launch_wgrad_bf16_rows(omoe_handle *h, cudaStream_t s, const CUtensorMap &a, const CUtensorMap &b, int M,
-                                   int N, int split, float *out0, float *out1);
+// Per matrix z < n_mat (1 or 2) and local expert e: C_z,e [M, N] (fp32) = A_z[seg_e]^T * B[seg_e], seg_e = the expert's rows
+// rounded up to 64.  a*, b: row-major activations [rows_cap, M or N] bf16 with a box of 64 rows; o*: [e_local, M, N] fp32 with
+// a box of 32 x 32.  Rows past an expert's count must be zero in A and finite in B.  (experts_sm100_wgrad.cu)
+struct alignas(64) WgradMaps {
+    CUtensorMap a0, a1, b, o0, o1;
+};
+cudaError_t launch_wgrad(omoe_handle *h, cudaStream_t s, const WgradMaps &maps, int n_mat, int M, int N);
 
 }  // namespace omoe

@@ -466,15 +466,6 @@ bool encode_map_bf16(CUtensorMap *m, void *ptr, uint64_t rows, uint64_t cols, ui
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-cudaError_t launch_grouped_plain(omoe_handle *h, cudaStream_t s, const CUtensorMap &a, const CUtensorMap &b,
-                                 const CUtensorMap &c, int n_out, int K) {
-    cudaError_t e = set_smem_attrs();
-    if (e != cudaSuccess) return e;
-    static int band = getenv("OMOE_BAND_DOWN") ? atoi(getenv("OMOE_BAND_DOWN")) : 16;
-    return launch_ex(grouped_gemm_kernel<false>, dim3(h->sm_count), dim3(kThreads), kSmemBytes, s, false, a, b, b, c,
-                     n_out, K, h->ex_tile_expert, h->ex_poffsets, h->e_local, band, h->dev_err, EpGate{});
-}
-
 // most 128-row tiles any placement of rows_ub rows on the local experts can give (-1: unknown)
 static long m_tiles_bound(omoe_handle *h, long rows_ub) {
     if (rows_ub < 0) return -1;

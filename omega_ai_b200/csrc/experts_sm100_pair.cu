@@ -300,8 +300,13 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                         for (int i = 0; i < 16; i++) {
                             // a gate lane finishes token 2i, its up lane token 2i + 1
                             const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[2 * i] : r[2 * i + 1], 8);
-                            const float g = __uint_as_float(up ? got : r[2 * i]);
-                            const float u = __uint_as_float(up ? r[2 * i + 1] : got);
+                            float g = __uint_as_float(up ? got : r[2 * i]);
+                            float u = __uint_as_float(up ? r[2 * i + 1] : got);
+                            if constexpr (KIND == PairKind::kUpGateKeep) {
+                                // h follows from the g and u that are kept: what the backward differentiates
+                                g = __bfloat162float(__float2bfloat16_rn(g));
+                                u = __bfloat162float(__float2bfloat16_rn(u));
+                            }
                             v[i] = o == 0 ? silu_f(g) * u : (o == 1 ? g : u);
                         }
 #pragma unroll

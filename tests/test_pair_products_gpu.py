@@ -23,3 +23,23 @@ def test_forward_at_tile_edges(oracle, T, d, dff, E, k):
     y, routing, logits, _ = run_gpu(xb, w_rb, rb(w_g), rb(w_u), rb(w_d), None, k, torch.bfloat16, torch.bfloat16)
     check_routing(routing, logits, r)
     assert_close_bf16(y, r.y)
+
+
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 64, 255, 256, 257, 481])
+def test_training_step_at_tile_edges(oracle, T):
+    """Both experts hold all T rows (top-2 of 2), so T is the width that the token tiles are cut from and the length the
+    weight gradients reduce over."""
+    from helpers import assert_close_bf16_grad
+    from test_backward_gpu import NAMES, run_layer
+    d, dff, E, k = 136, 328, 2, 2
+    x, w_r, w_g, w_u, w_d, _ = make_layer(T, d, dff, E, k, seed=T)
+    rb = oracle.bf16_round
+    x, w_r, w_g, w_u, w_d = rb(x), rb(w_r * 10), rb(w_g * 3), rb(w_u * 3), rb(w_d * 3)
+    dy = rb(np.random.default_rng(T).standard_normal((T, d)).astype(np.float32))
+    got, routing = run_layer(T, d, dff, E, k, torch.bfloat16, torch.bfloat16, x, w_r, w_g, w_u, w_d, dy)
+    r = oracle.moe_forward(x, w_r, w_g, w_u, w_d, k, bf16=True)
+    assert np.array_equal(routing[0], r.topk_idx)
+    assert_close_bf16_grad(got["y"], r.y)
+    ref = oracle.moe_backward(x, w_r, w_g, w_u, w_d, k, dy, bf16=True, out_bf16=True)
+    for name in NAMES:
+        assert_close_bf16_grad(got[name], getattr(ref, name))
