@@ -167,7 +167,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
 
     if (warp == 0) {
         // ---------------- producer ----------------
-        if (lane == 0) {
+        {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -178,28 +178,31 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 const int small = b_rows > 64 ? 0 : (b_rows + 31) / 32;  // 32-row boxes instead of one of 128 rows
                 const uint32_t bytes = kABytesP + (small ? small * 4096 : 16384);
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
-                    const uint32_t sa = base + stage * kStageBytesP, sb = sa + kABytesP;
-                    const uint32_t bar = map_to_rank(full_bar(stage), 0);
-                    if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * bytes);
-                    const bool second = KIND == PairKind::kPlainMN2 && kb >= kb_src;
-                    const int kx = (second ? kb - kb_src : kb) * BLOCK_K;
-                    if constexpr (kGate) {
-                        pair_load_4d(sa, &maps.a0, bar, kx, 0, 0, (t.e * n_out + t.ft * 128 + (int)rank * 64) >> 3);
-                    } else if constexpr (!kMN) {
-                        pair_load_2d(sa, &maps.a0, bar, kx, t.e * n_out + t.ft * 256 + (int)rank * 128);
-                    } else {
-                        const CUtensorMap *ma = second ? &maps.a1 : &maps.a0;
-                        const int x = t.ft * 256 + (int)rank * 128;
-                        pair_load_3d(sa, ma, bar, x, kx, t.e);
-                        pair_load_3d(sa + 8192, ma, bar, x + 64, kx, t.e);
+                    if (!warp_wait(empty_bar(stage), phase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
+                    if (elect_one()) {
+                        const uint32_t sa = base + stage * kStageBytesP, sb = sa + kABytesP;
+                        const uint32_t bar = map_to_rank(full_bar(stage), 0);
+                        if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * bytes);
+                        const bool second = KIND == PairKind::kPlainMN2 && kb >= kb_src;
+                        const int kx = (second ? kb - kb_src : kb) * BLOCK_K;
+                        if constexpr (kGate) {
+                            pair_load_4d(sa, &maps.a0, bar, kx, 0, 0, (t.e * n_out + t.ft * 128 + (int)rank * 64) >> 3);
+                        } else if constexpr (!kMN) {
+                            pair_load_2d(sa, &maps.a0, bar, kx, t.e * n_out + t.ft * 256 + (int)rank * 128);
+                        } else {
+                            const CUtensorMap *ma = second ? &maps.a1 : &maps.a0;
+                            const int x = t.ft * 256 + (int)rank * 128;
+                            pair_load_3d(sa, ma, bar, x, kx, t.e);
+                            pair_load_3d(sa + 8192, ma, bar, x + 64, kx, t.e);
+                        }
+                        if (small == 0) {
+                            pair_load_2d(sb, second ? &maps.b1 : &maps.b0, bar, kx, row_b);
+                        } else {
+                            const CUtensorMap *mb = second ? &maps.b1_32 : &maps.b0_32;
+                            for (int i = 0; i < small; i++) pair_load_2d(sb + i * 4096, mb, bar, kx, row_b + i * 32);
+                        }
                     }
-                    if (small == 0) {
-                        pair_load_2d(sb, second ? &maps.b1 : &maps.b0, bar, kx, row_b);
-                    } else {
-                        const CUtensorMap *mb = second ? &maps.b1_32 : &maps.b0_32;
-                        for (int i = 0; i < small; i++) pair_load_2d(sb + i * 4096, mb, bar, kx, row_b + i * 32);
-                    }
+                    __syncwarp();
                     if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -211,7 +214,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (even CTA, for both) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             int stage = 0, as = 0;
             uint32_t phase = 0, aphase = 0;
             bool ok = true;
@@ -219,23 +222,27 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 const PairTile t = tile_at(tile);
                 const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (kMN ? 1u << 15 : 0u) |
                                        ((uint32_t)(t.n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
-                if (!mbar_wait(tempty_bar(as), aphase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
+                if (!warp_wait(tempty_bar(as), aphase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * kTokensMax;
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag, dev_err)) { ok = false; break; }
+                    if (!warp_wait(full_bar(stage), phase, abort_flag, dev_err)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = base + stage * kStageBytesP;
                     const uint64_t adesc = kMN ? make_mn_desc(sa) : make_sw128_desc(sa);
                     const uint64_t bdesc = make_sw128_desc(sa + kABytesP);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BLOCK_K / UMMA_K; k++)  // 16 of the reduction: 32 bytes on, or 16 rows of 128 bytes
-                        pair_mma_bf16(d_tmem, adesc + (kMN ? 128u : 2u) * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                    pair_commit(empty_bar(stage));
+                        for (int k = 0; k < BLOCK_K / UMMA_K; k++)  // 16 of the reduction: 32 bytes on, or 16 rows of 128 bytes
+                            pair_mma_bf16(d_tmem, adesc + (kMN ? 128u : 2u) * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        pair_commit(empty_bar(stage));
+                    }
+                    __syncwarp();
                     if (++stage == kStagesP) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                pair_commit(tfull_bar(as));
+                if (elect_one()) pair_commit(tfull_bar(as));
+                __syncwarp();
                 if (++as == kAccStagesP) { as = 0; aphase ^= 1u; }
             }
         }

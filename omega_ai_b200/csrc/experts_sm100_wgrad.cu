@@ -106,7 +106,7 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
 
     if (warp == 0) {
         // ---------------- producer ----------------
-        if (lane == 0) {
+        {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -117,16 +117,19 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
                 const CUtensorMap *ma = t.z ? &maps.a1 : &maps.a0;
                 const int xa = t.mt * 256 + (int)rank * 128, xb = t.nt * 256 + (int)rank * 128;
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
-                    const uint32_t sa = base + stage * kStageBytesW;
-                    const uint32_t bar = map_to_rank(full_bar(stage), 0);
-                    const int y = seg0 + kb * BLOCK_K;
-                    if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * kStageBytesW);
+                    if (!warp_wait(empty_bar(stage), phase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
+                    if (elect_one()) {
+                        const uint32_t sa = base + stage * kStageBytesW;
+                        const uint32_t bar = map_to_rank(full_bar(stage), 0);
+                        const int y = seg0 + kb * BLOCK_K;
+                        if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * kStageBytesW);
 #pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        pair_load_2d(sa + i * kBoxBytesW, ma, bar, xa + 64 * i, y);
-                        pair_load_2d(sa + kABytesW + i * kBoxBytesW, &maps.b, bar, xb + 64 * i, y);
+                        for (int i = 0; i < 2; i++) {
+                            pair_load_2d(sa + i * kBoxBytesW, ma, bar, xa + 64 * i, y);
+                            pair_load_2d(sa + kABytesW + i * kBoxBytesW, &maps.b, bar, xb + 64 * i, y);
+                        }
                     }
+                    __syncwarp();
                     if (++stage == kStagesW) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -138,7 +141,7 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (even CTA, for both) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                                        ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
             int stage = 0, as = 0;
@@ -147,23 +150,27 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
             for (int tile = pair0; ok && tile < total; tile += pairs) {
                 const WTile t = wtile(tile, E, m_tiles, n_tiles);
                 const int num_kb = (counts[t.e] + BLOCK_K - 1) / BLOCK_K;
-                if (!mbar_wait(tempty_bar(as), aphase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
+                if (!warp_wait(tempty_bar(as), aphase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * 256;
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!mbar_wait(full_bar(stage), phase, abort_flag, dev_err)) { ok = false; break; }
+                    if (!warp_wait(full_bar(stage), phase, abort_flag, dev_err)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = base + stage * kStageBytesW;
                     const uint64_t adesc = make_mn_desc(sa), bdesc = make_mn_desc(sa + kABytesW);
                     // 16 rows of the reduction are 16 x 128 bytes further on: +128 in 16-byte units
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < BLOCK_K / UMMA_K; k++)
-                        pair_mma_bf16(d_tmem, adesc + 128u * k, bdesc + 128u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                    pair_commit(empty_bar(stage));
+                        for (int k = 0; k < BLOCK_K / UMMA_K; k++)
+                            pair_mma_bf16(d_tmem, adesc + 128u * k, bdesc + 128u * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        pair_commit(empty_bar(stage));
+                    }
+                    __syncwarp();
                     if (++stage == kStagesW) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                pair_commit(tfull_bar(as));  // accumulator complete (at once for an expert without rows)
+                if (elect_one()) pair_commit(tfull_bar(as));  // accumulator complete (at once for an expert without rows)
+                __syncwarp();
                 if (++as == kAccStagesW) { as = 0; aphase ^= 1u; }
             }
         }

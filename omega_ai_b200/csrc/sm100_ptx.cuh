@@ -69,6 +69,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// One lane of a converged warp.  The TMA and tcgen05 instructions of a role take their operands from uniform registers: a
+// role that runs as a whole warp and elects a lane around each of them keeps its descriptors and barrier addresses there,
+// where a branch on the lane number makes the compiler move every operand over again for each instruction.  Measured on the
+// pair kernel's issue loop with the loads and the epilogue taken out: 650 cycles per 64-deep k-block whatever its width
+// (its four MMAs take 508) with the branch, the MMAs' own time with the election.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// mbar_wait by a whole converged warp: the same answer in every lane.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int32_t *dev_err) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, dev_err));
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
