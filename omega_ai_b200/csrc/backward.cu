@@ -22,7 +22,7 @@
 // memory and three passes over the weights after every omoe_set_weights.  The weight-gradient products reduce over an
 // expert's rows and read the activations in place; padding rows are zeroed in xp and dyp, hence zero in everything
 // derived from them.
-// fp32 layers: a plain tiled FMA kernel with strided operands (sized for parity runs, not for speed).
+// fp32 layers: the CUDA-core products of experts_f32.cu, which skip padding rows.
 #include <stdlib.h>
 #include <string.h>
 
@@ -75,22 +75,6 @@ __device__ __forceinline__ float silu_grad_f32(float x) {
 }
 
 // ---- element-wise passes over the rows in use -----------------------------------------------------
-// h = silu(g) * u for rows [0, *rows_in_use); gu is [rows, 2*dff] with g in the left half.
-template <typename T>
-__global__ void __launch_bounds__(256)
-swiglu_fwd_kernel(const T *__restrict__ gu, T *__restrict__ h, const int32_t *__restrict__ rows_in_use, int dff) {
-    const int64_t vec = dff / 8, total = (int64_t)*rows_in_use * vec;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / vec, c = (i % vec) * 8;
-        float g[8], u[8], o[8];
-        load8(gu + r * 2 * dff + c, g);
-        load8(gu + r * 2 * dff + dff + c, u);
-#pragma unroll
-        for (int j = 0; j < 8; j++) o[j] = silu_f32(g[j]) * u[j];
-        store8(h + r * dff + c, o);
-    }
-}
-
 // dg = (dh * u) * silu'(g), du = dh * silu(g); dgu is [rows, 2*dff] with dg in the left half.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -330,98 +314,17 @@ __global__ void __launch_bounds__(256) dbias_kernel(const float *__restrict__ dl
 }
 
 // Zero the padding rows of every expert's segment (rows [poffsets[e] + counts[e], poffsets[e+1])) of buf
-// [rows, ld] (16-byte vectors; ld*sizeof(T) is a multiple of 16).  blockIdx.x = expert.
-template <typename T>
+// [rows, ld] (16-byte vectors; ld is a multiple of 8).  blockIdx.x = expert.
 __global__ void __launch_bounds__(256)
-zero_pad_rows_kernel(T *__restrict__ buf, int ld, const int32_t *__restrict__ poffsets,
+zero_pad_rows_kernel(__nv_bfloat16 *__restrict__ buf, int ld, const int32_t *__restrict__ poffsets,
                      const int32_t *__restrict__ counts) {
     const int e = blockIdx.x;
     const int r0 = poffsets[e] + counts[e], r1 = poffsets[e + 1];
-    const int vec_per_row = ld * (int)sizeof(T) / 16;
+    const int vec_per_row = ld / 8;
     const int64_t total = (int64_t)(r1 - r0) * vec_per_row;
     uint4 *base = reinterpret_cast<uint4 *>(buf + (size_t)r0 * ld);
     for (int64_t i = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.y * blockDim.x)
         base[i] = make_uint4(0u, 0u, 0u, 0u);
-}
-
-// ---- fp32 products (parity-sized) -----------------------------------------------------------------
-// Rows grouped by expert: C[r, n] (+)= sum_k A[r, k] * B_e(k, n) for the rows in use, where the expert of
-// a row comes from its 128-row tile and B_e(k, n) = B[e*sbe + k*sbk + n*sbn].  64 x 64 tiles, 4 x 4 per thread.
-__global__ void __launch_bounds__(256)
-sgemm_rows_kernel(const float *__restrict__ A, int lda, const float *__restrict__ B, size_t sbe, int sbk, int sbn,
-                  float *__restrict__ Cm, int ldc, int N, int K, const int32_t *__restrict__ rows_in_use,
-                  const int32_t *__restrict__ tile_expert, int accumulate) {
-    __shared__ float sa[16][65], sb[16][65];
-    const int r0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
-    if (r0 >= *rows_in_use) return;
-    const int e = tile_expert[r0 / kRowAlign];
-    const float *Be = B + (size_t)e * sbe;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-            const int kk = i & 15, m = i >> 4;
-            sa[kk][m] = (k0 + kk < K) ? A[(size_t)(r0 + m) * lda + k0 + kk] : 0.f;
-            const int n = n0 + m;
-            sb[kk][m] = (k0 + kk < K && n < N) ? Be[(size_t)(k0 + kk) * sbk + (size_t)n * sbn] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) { a[i] = sa[kk][ty * 4 + i]; b[i] = sb[kk][tx * 4 + i]; }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) {
-            const int r = r0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (n < N) {
-                float *p = Cm + (size_t)r * ldc + n;
-                *p = accumulate ? *p + acc[i][j] : acc[i][j];
-            }
-        }
-}
-
-// Weight gradient of one expert (blockIdx.z): C_e[m, n] = sum over the expert's rows r of A[r, m] * B[r, n].
-__global__ void __launch_bounds__(256)
-sgemm_wgrad_kernel(const float *__restrict__ A, int lda, const float *__restrict__ B, int ldb, float *__restrict__ Cm,
-                   int M, int N, const int32_t *__restrict__ poffsets, const int32_t *__restrict__ counts) {
-    __shared__ float sa[16][65], sb[16][65];
-    const int e = blockIdx.z, m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int row0 = poffsets[e], cnt = counts[e];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < cnt; k0 += 16) {
-        for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-            const int kk = i >> 6, m = i & 63;
-            const bool in = k0 + kk < cnt;
-            sa[kk][m] = (in && m0 + m < M) ? A[(size_t)(row0 + k0 + kk) * lda + m0 + m] : 0.f;
-            sb[kk][m] = (in && n0 + m < N) ? B[(size_t)(row0 + k0 + kk) * ldb + n0 + m] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) { a[i] = sa[kk][ty * 4 + i]; b[i] = sb[kk][tx * 4 + i]; }
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < N) Cm[((size_t)e * M + m) * N + n] = acc[i][j];
-        }
 }
 
 int grid_for(int64_t work_items, int sm_count) {
@@ -436,46 +339,17 @@ int grid_for(int64_t work_items, int sm_count) {
         if (_e != cudaSuccess) return _e;             \
     } while (0)
 
-template <typename CT>
-cudaError_t forward_experts_t(omoe_handle *h, BwState *b, cudaStream_t s, int *n) {
-    const int d = h->cfg.d_model, dff = h->cfg.d_ff, El = h->e_local;
-    const int32_t *rows_in_use = h->ex_poffsets + El;
-    CT *gu = static_cast<CT *>(b->gu);
+cudaError_t forward_experts(omoe_handle *h, BwState *b, cudaStream_t s, int *n) {
+    const int d = h->cfg.d_model, dff = h->cfg.d_ff;
+    if (h->cfg.compute_dtype != OMOE_BF16) return f32_forward_experts(h, s, b->gu, n);
     // padding rows hold rows of earlier steps: zero them, so that g, u and h are zero there too and a
-    // reduction over a padded segment (the weight gradients) adds nothing
-    zero_pad_rows_kernel<CT><<<dim3(El, 8), 256, 0, s>>>(static_cast<CT *>(h->xp), d, h->ex_poffsets, h->ex_counts);
+    // reduction over blocks of 64 rows (the weight gradients) adds nothing
+    zero_pad_rows_kernel<<<dim3(h->e_local, 8), 256, 0, s>>>(static_cast<__nv_bfloat16 *>(h->xp), d, h->ex_poffsets,
+                                                             h->ex_counts);
     BW_TRY(cudaGetLastError());
-    (*n)++;
-    if constexpr (sizeof(CT) == 2) {
-        BW_TRY(launch_pair(h, s, false, PairKind::kUpGateKeep, b->up, dff, d, 64));
-        (*n)++;
-    } else {
-        dim3 grid((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(dff, 64));
-        const float *xp = static_cast<const float *>(h->xp);
-        // g[r, f] = sum_c xp[r, c] * Wg[e][f][c]
-        sgemm_rows_kernel<<<grid, 256, 0, s>>>(xp, d, static_cast<const float *>(h->w_gate), (size_t)dff * d, 1, d,
-                                               reinterpret_cast<float *>(gu), 2 * dff, dff, d, rows_in_use,
-                                               h->ex_tile_expert, 0);
-        sgemm_rows_kernel<<<grid, 256, 0, s>>>(xp, d, static_cast<const float *>(h->w_up), (size_t)dff * d, 1, d,
-                                               reinterpret_cast<float *>(gu) + dff, 2 * dff, dff, d, rows_in_use,
-                                               h->ex_tile_expert, 0);
-        swiglu_fwd_kernel<CT><<<grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count), 256, 0, s>>>(
-            gu, static_cast<CT *>(h->hbuf), rows_in_use, dff);
-        BW_TRY(cudaGetLastError());
-        *n += 3;
-    }
-    if constexpr (sizeof(CT) == 2) {
-        BW_TRY(launch_pair(h, s, false, PairKind::kPlain, h->maps.down, d, dff, 32));
-    } else {
-        dim3 grid((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(d, 64));
-        // yp[r, c] = sum_f h[r, f] * Wd[e][c][f]
-        sgemm_rows_kernel<<<grid, 256, 0, s>>>(static_cast<const float *>(h->hbuf), dff,
-                                               static_cast<const float *>(h->w_down), (size_t)dff * d, 1, dff,
-                                               static_cast<float *>(h->yp), d, d, dff, rows_in_use, h->ex_tile_expert,
-                                               0);
-        BW_TRY(cudaGetLastError());
-    }
-    (*n)++;
+    BW_TRY(launch_pair(h, s, false, PairKind::kUpGateKeep, b->up, dff, d, 64));
+    BW_TRY(launch_pair(h, s, false, PairKind::kPlain, h->maps.down, d, dff, 32));
+    *n += 3;
     return cudaSuccess;
 }
 
@@ -506,11 +380,11 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
         BW_TRY(ep_wait_rows(h, s));  // every rank's gradient rows for my experts have landed
         (*n)++;
     }
-    zero_pad_rows_kernel<CT><<<dim3(El, 8), 256, 0, s>>>(static_cast<CT *>(b->dyp), d, h->ex_poffsets, h->ex_counts);
-    BW_TRY(cudaGetLastError());
-    (*n)++;
-    const int ew_grid = grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count);
     if constexpr (sizeof(CT) == 2) {
+        zero_pad_rows_kernel<<<dim3(El, 8), 256, 0, s>>>(static_cast<CT *>(b->dyp), d, h->ex_poffsets, h->ex_counts);
+        BW_TRY(cudaGetLastError());
+        (*n)++;
+        const int ew_grid = grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count);
         // dh = dyp * W_down; rows up to a multiple of 64, because the weight gradients reduce over blocks of 64 rows
         BW_TRY(launch_pair(h, s, false, PairKind::kPlainMN, b->dh_maps, dff, d, 64));
         (*n)++;
@@ -530,35 +404,16 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
         BW_TRY(launch_wgrad(h, s, b->w_gu, 2, dff, d));
         *n += 2;
     } else {
-        const float *dyp = static_cast<const float *>(b->dyp);
-        float *dgu = static_cast<float *>(b->dgu);
-        dim3 g1((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(dff, 64));
-        // dh[r, f] = sum_c dyp[r, c] * Wd[e][c][f]
-        sgemm_rows_kernel<<<g1, 256, 0, s>>>(dyp, d, static_cast<const float *>(h->w_down), (size_t)dff * d, dff, 1,
-                                             static_cast<float *>(b->dh), dff, dff, d, rows_in_use, h->ex_tile_expert,
-                                             0);
-        swiglu_bwd_kernel<CT><<<ew_grid, 256, 0, s>>>(static_cast<const CT *>(b->dh), static_cast<const CT *>(b->gu),
-                                                      static_cast<CT *>(b->dgu), rows_in_use, dff);
-        dim3 g2((unsigned)(h->rows_cap / 64), (unsigned)ceil_div(d, 64));
-        // dxp[r, c] = sum_f dg[r, f] * Wg[e][f][c] + sum_f du[r, f] * Wu[e][f][c]
-        sgemm_rows_kernel<<<g2, 256, 0, s>>>(dgu, 2 * dff, static_cast<const float *>(h->w_gate), (size_t)dff * d, d, 1,
-                                             static_cast<float *>(b->dxp), d, d, dff, rows_in_use, h->ex_tile_expert, 0);
-        sgemm_rows_kernel<<<g2, 256, 0, s>>>(dgu + dff, 2 * dff, static_cast<const float *>(h->w_up), (size_t)dff * d,
-                                             d, 1, static_cast<float *>(b->dxp), d, d, dff, rows_in_use,
-                                             h->ex_tile_expert, 1);
+        // dg | du from dyp * W_down, then dxp = dg * W_gate + du * W_up
+        BW_TRY(f32_grad_rows(h, s, b->dyp, b->gu, b->dgu, b->dxp, n));
         if (ep) {
             BW_TRY(ep_signal_out(h, s));
             (*n)++;
         }
-        // d W_down[e][c][f] = sum_r dyp[r, c] * h[r, f];  d W_gate[e][f][c] = sum_r dg[r, f] * xp[r, c]
-        sgemm_wgrad_kernel<<<dim3(ceil_div(dff, 64), ceil_div(d, 64), El), 256, 0, s>>>(
-            dyp, d, static_cast<const float *>(h->hbuf), dff, b->d_down, d, dff, h->ex_poffsets, h->ex_counts);
-        sgemm_wgrad_kernel<<<dim3(ceil_div(d, 64), ceil_div(dff, 64), El), 256, 0, s>>>(
-            dgu, 2 * dff, static_cast<const float *>(h->xp), d, b->d_gate, dff, d, h->ex_poffsets, h->ex_counts);
-        sgemm_wgrad_kernel<<<dim3(ceil_div(d, 64), ceil_div(dff, 64), El), 256, 0, s>>>(
-            dgu + dff, 2 * dff, static_cast<const float *>(h->xp), d, b->d_up, dff, d, h->ex_poffsets, h->ex_counts);
-        BW_TRY(cudaGetLastError());
-        *n += 7;
+        // d W_down[e][c][f] = sum_r dyp[r, c] * h[r, f];  d W_gate[e][f][c], d W_up = sum_r dg[r, f], du[r, f] * xp[r, c]
+        BW_TRY(f32_wgrad(h, s, b->dyp, d, 0, h->hbuf, 1, d, dff, b->d_down, nullptr));
+        BW_TRY(f32_wgrad(h, s, b->dgu, 2 * dff, dff, h->xp, 2, dff, d, b->d_gate, b->d_up));
+        *n += 2;
     }
     // router: d W_router = dl^T * x, d bias = column sums of dl
     {
@@ -710,8 +565,7 @@ void bw_forward_empty(omoe_handle *h) {
 
 cudaError_t bw_forward_experts(omoe_handle *h, int T, cudaStream_t s, int *n) {
     BwState *b = static_cast<BwState *>(h->bw);
-    cudaError_t e = h->cfg.compute_dtype == OMOE_BF16 ? forward_experts_t<__nv_bfloat16>(h, b, s, n)
-                                                      : forward_experts_t<float>(h, b, s, n);
+    cudaError_t e = forward_experts(h, b, s, n);
     b->fwd_valid = e == cudaSuccess;
     b->fwd_T = T;
     return e;
