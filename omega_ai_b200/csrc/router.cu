@@ -215,31 +215,48 @@ router_kernel(const XT *__restrict__ x, const WT *__restrict__ w_r, const float 
         if constexpr (S == 1) __syncthreads();
     }
 
-    // xor butterfly over all accumulators first (independent chains overlap), then lane (e % 32) publishes logit e
-    float red[TPW][EPW];
+    // Sum over the lanes: an xor tree over 16, 8, 4, 2, 1.  Every lane of a butterfly ends with the same sum, so a lane
+    // needs only the values it will publish: at each step it keeps one half of its values and hands the other half to
+    // its partner (fp32 addition commutes, so every sum has the butterfly's bits).  NV values take about NV exchanges
+    // this way, not 5 NV: with 4 tokens x 16 experts per warp 62 shuffles for 320.
+    constexpr int NV = TPW * EPW;
+    float red[NV];
 #pragma unroll
     for (int i = 0; i < TPW; i++)
 #pragma unroll
         for (int e = 0; e < EPW; e++)
-            red[i][e] = __uint_as_float((uint32_t)acc[i][e]) + __uint_as_float((uint32_t)(acc[i][e] >> 32));  // even + odd
+            red[i * EPW + e] = __uint_as_float((uint32_t)acc[i][e]) + __uint_as_float((uint32_t)(acc[i][e] >> 32));  // even + odd
 #pragma unroll
-    for (int m = 16; m >= 1; m >>= 1)
+    for (int st = 0; st < 5; st++) {
+        const int m = 16 >> st;
+        const int cur = NV >> st;  // values a lane still holds
+        if (cur >= 2) {
+            const bool hi = lane & m;
 #pragma unroll
-        for (int i = 0; i < TPW; i++)
+            for (int i = 0; i < cur / 2; i++) {
+                const float send = hi ? red[i] : red[i + cur / 2];
+                const float keep = hi ? red[i + cur / 2] : red[i];
+                red[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+            }
+        } else {
+            red[0] = red[0] + __shfl_xor_sync(0xffffffffu, red[0], m);
+        }
+    }
+    constexpr int HELD = NV >= 32 ? NV / 32 : 1;    // values of a lane: HELD * (lane / DUP) + j
+    constexpr int DUP = NV >= 32 ? 1 : 32 / NV;     // neighbouring lanes with the same value
+    if (lane % DUP == 0) {
 #pragma unroll
-            for (int e = 0; e < EPW; e++) red[i][e] = red[i][e] + __shfl_xor_sync(0xffffffffu, red[i][e], m);
-#pragma unroll
-    for (int i = 0; i < TPW; i++)
-#pragma unroll
-        for (int e = 0; e < EPW; e++) {
-            const int eg = es * EPW + e, tt = grp * TPW + i;
-            if (lane == (e & 31) && eg < E) {
-                float v = red[i][e];
+        for (int j = 0; j < HELD; j++) {
+            const int vi = (lane / DUP) * HELD + j;
+            const int eg = es * EPW + vi % EPW, tt = grp * TPW + vi / EPW;
+            if (eg < E) {
+                float v = red[j];
                 if (bias != nullptr) v = v + sbias[eg];
                 sl[tt * EMAX + eg] = v;
                 if (t0 + tt < T) logits[(size_t)(t0 + tt) * E + eg] = v;
             }
         }
+    }
     __syncthreads();
 
     // Softmax statistics, top-k on the logits, gate weights: a group of GW lanes per token
