@@ -27,6 +27,7 @@
 #include <string.h>
 
 #include <new>
+#include <type_traits>
 
 #include "backward.cuh"
 #include "common.cuh"
@@ -62,11 +63,6 @@ struct BwState {
 
 namespace {
 
-// ---- element access for fp32 and bf16 rows --------------------------------------------------------
-__device__ __forceinline__ float ldf(const float *p) { return *p; }
-__device__ __forceinline__ float ldf(const __nv_bfloat16 *p) { return __bfloat162float(*p); }
-
-
 __device__ __forceinline__ float silu_f32(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float silu_grad_f32(float x) {
     const float sg = 1.0f / (1.0f + expf(-x));
@@ -79,6 +75,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const T *__restrict__ dh, const T *__restrict__ gu, T *__restrict__ dgu,
                   const int32_t *__restrict__ rows_in_use, int dff) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t vec = dff / 8, total = (int64_t)*rows_in_use * vec;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / vec, c = (i % vec) * 8;
@@ -109,6 +107,8 @@ combine_bwd_kernel(const OT *__restrict__ dy, void *const *__restrict__ yp_table
                    const float *__restrict__ topk_w, const float *__restrict__ logits, float *__restrict__ dgw,
                    float *__restrict__ dl, int T, int d, int k, int E, int renorm, float aux_c,
                    const int32_t *__restrict__ counts) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t < T) {
@@ -222,6 +222,8 @@ __global__ void __launch_bounds__(256)
 dx_kernel(void *const *__restrict__ dxp_table, int e_local, const int32_t *__restrict__ topk_idx, EpWait wait,
           int32_t *dev_err, const int32_t *__restrict__ pos, const float *__restrict__ dl,
           const float *__restrict__ w_r, OT *__restrict__ dx, int T, int d, int k, int E) {
+    pdl_trigger();
+    pdl_wait();
     extern __shared__ float s_dl[];  // [warps][E]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -279,6 +281,8 @@ template <typename XT>
 __global__ void __launch_bounds__(256)
 dwr_partial_kernel(const XT *__restrict__ x, const float *__restrict__ dl, float *__restrict__ part, int T, int d,
                    int E, int slices) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float s_dl[kDwrTokens][kDwrExperts];
     const int c = blockIdx.x * 512 + threadIdx.x * 2;
     const int e0 = blockIdx.z * kDwrExperts;
@@ -321,6 +325,8 @@ dwr_partial_kernel(const XT *__restrict__ x, const float *__restrict__ dl, float
 
 __global__ void __launch_bounds__(256)
 dwr_reduce_kernel(const float *__restrict__ part, float *__restrict__ out, int n, int slices) {
+    pdl_trigger();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float acc = 0.f;
@@ -331,6 +337,8 @@ dwr_reduce_kernel(const float *__restrict__ part, float *__restrict__ out, int n
 
 // d bias[e] = sum_t dl[t, e]: one block per expert, threads stride the tokens, fixed tree at the end.
 __global__ void __launch_bounds__(256) dbias_kernel(const float *__restrict__ dl, float *__restrict__ out, int T, int E) {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float s[256];
     const int e = blockIdx.x;
     float acc = 0.f;
@@ -349,6 +357,8 @@ __global__ void __launch_bounds__(256) dbias_kernel(const float *__restrict__ dl
 __global__ void __launch_bounds__(256)
 zero_pad_rows_kernel(__nv_bfloat16 *__restrict__ buf, int ld, const int32_t *__restrict__ poffsets,
                      const int32_t *__restrict__ counts) {
+    pdl_trigger();
+    pdl_wait();
     const int e = blockIdx.x;
     const int r0 = poffsets[e] + counts[e], r1 = poffsets[e + 1];
     const int vec_per_row = ld / 8;
@@ -370,16 +380,20 @@ int grid_for(int64_t work_items, int sm_count) {
         if (_e != cudaSuccess) return _e;             \
     } while (0)
 
+// Programmatic dependent launch along the training step, as along the forward (pdl.cuh): every kernel of it waits before its
+// first access.  One GPU only: with expert parallelism kernels without the instructions stand in between.
+bool bw_pdl(const omoe_handle *h) { return h->pdl && h->cfg.world == 1; }
+
 cudaError_t forward_experts(omoe_handle *h, BwState *b, cudaStream_t s, int *n) {
     const int d = h->cfg.d_model, dff = h->cfg.d_ff;
     if (h->cfg.compute_dtype != OMOE_BF16) return f32_forward_experts(h, s, b->gu, n);
     // padding rows hold rows of earlier steps: zero them, so that g, u and h are zero there too and a
     // reduction over blocks of 64 rows (the weight gradients) adds nothing
-    zero_pad_rows_kernel<<<dim3(h->e_local, 8), 256, 0, s>>>(static_cast<__nv_bfloat16 *>(h->xp), d, h->ex_poffsets,
-                                                             h->ex_counts);
-    BW_TRY(cudaGetLastError());
-    BW_TRY(launch_pair(h, s, false, PairKind::kUpGateKeep, b->up, dff, d, 64));
-    BW_TRY(launch_pair(h, s, false, PairKind::kPlain, h->maps.down, d, dff, 32));
+    const bool pdl = bw_pdl(h);
+    BW_TRY(launch_ex(zero_pad_rows_kernel, dim3(h->e_local, 8), dim3(256), 0, s, pdl, static_cast<__nv_bfloat16 *>(h->xp), d,
+                     h->ex_poffsets, h->ex_counts));
+    BW_TRY(launch_pair(h, s, pdl, PairKind::kUpGateKeep, b->up, dff, d, 64));
+    BW_TRY(launch_pair(h, s, pdl, PairKind::kPlain, h->maps.down, d, dff, 32));
     *n += 3;
     return cudaSuccess;
 }
@@ -390,7 +404,7 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
     const int d = h->cfg.d_model, dff = h->cfg.d_ff, El = h->e_local, E = h->cfg.n_experts, k = h->cfg.top_k;
     const int32_t *rows_in_use = h->ex_poffsets + El;
     const int warps = 8, tblocks = ceil_div(T, warps);
-    const bool ep = h->cfg.world > 1;
+    const bool ep = h->cfg.world > 1, pdl = bw_pdl(h);
     EpSignal sig{nullptr, 1, 0, nullptr};
     if (ep) {
         BW_TRY(ep_bw_advance(h, s));  // the backward is a step of its own for the flags
@@ -398,11 +412,9 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
         sig = ep_rows_signal(h);
     }
     if (T > 0) {
-        combine_bwd_kernel<CT, OT><<<tblocks, 256, 0, s>>>(
-            static_cast<const OT *>(dy), h->d_out_table, b->dyp_table, El, sig, h->ticket, h->pos, h->topk_idx,
+        BW_TRY(launch_ex(combine_bwd_kernel<CT, OT>, dim3(tblocks), dim3(256), 0, s, pdl, static_cast<const OT *>(dy), h->d_out_table, b->dyp_table, El, sig, h->ticket, h->pos, h->topk_idx,
             h->topk_w, h->logits, b->dgw, b->dl, T, d, k, E, h->cfg.renormalize,
-            b->aux_coef != 0.f ? b->aux_coef * (float)E / (float)T : 0.f, h->counts);
-        BW_TRY(cudaGetLastError());
+            b->aux_coef != 0.f ? b->aux_coef * (float)E / (float)T : 0.f, h->counts));
     } else {
         BW_TRY(ep_signal_rows(h, s));  // no tokens here: nothing to send, but the owners wait for every rank
     }
@@ -412,18 +424,17 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
         (*n)++;
     }
     if constexpr (sizeof(CT) == 2) {
-        zero_pad_rows_kernel<<<dim3(El, 8), 256, 0, s>>>(static_cast<CT *>(b->dyp), d, h->ex_poffsets, h->ex_counts);
-        BW_TRY(cudaGetLastError());
+        BW_TRY(launch_ex(zero_pad_rows_kernel, dim3(El, 8), dim3(256), 0, s, pdl, static_cast<CT *>(b->dyp), d, h->ex_poffsets,
+                         h->ex_counts));
         (*n)++;
         const int ew_grid = grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count);
         // dh = dyp * W_down; rows up to a multiple of 64, because the weight gradients reduce over blocks of 64 rows
-        BW_TRY(launch_pair(h, s, false, PairKind::kPlainMN, b->dh_maps, dff, d, 64));
+        BW_TRY(launch_pair(h, s, pdl, PairKind::kPlainMN, b->dh_maps, dff, d, 64));
         (*n)++;
-        swiglu_bwd_kernel<CT><<<ew_grid, 256, 0, s>>>(static_cast<const CT *>(b->dh), static_cast<const CT *>(b->gu),
-                                                      static_cast<CT *>(b->dgu), rows_in_use, dff);
-        BW_TRY(cudaGetLastError());
+        BW_TRY(launch_ex(swiglu_bwd_kernel<CT>, dim3(ew_grid), dim3(256), 0, s, pdl, static_cast<const CT *>(b->dh),
+                         static_cast<const CT *>(b->gu), static_cast<CT *>(b->dgu), rows_in_use, dff));
         (*n)++;
-        BW_TRY(launch_pair(h, s, false, PairKind::kPlainMN2, b->dxp_maps, d, dff, 32));
+        BW_TRY(launch_pair(h, s, pdl, PairKind::kPlainMN2, b->dxp_maps, d, dff, 32));
         (*n)++;
         if (ep) {
             // the input-gradient rows are complete: the token ranks may fetch them while the weight gradients run
@@ -450,20 +461,21 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
     {
         const int slices = b->dwr_slices;
         dim3 grid((unsigned)ceil_div(d, 512), (unsigned)slices, (unsigned)ceil_div(E, kDwrExperts));
-        auto run = [&](auto *xr) { dwr_partial_kernel<<<grid, 256, 0, s>>>(xr, b->dl, b->dwr_part, T, d, E, slices); };
+        auto run = [&](auto *xr) {
+            using XT = typename std::remove_cv<typename std::remove_pointer<decltype(xr)>::type>::type;
+            return launch_ex(dwr_partial_kernel<XT>, grid, dim3(256), 0, s, pdl, xr, b->dl, b->dwr_part, T, d, E, slices);
+        };
         // x: the rows the router saw (the caller's rows, or the normalised rows of the block form)
-        if (x_is_compute) run(static_cast<const CT *>(x));
-        else run(static_cast<const OT *>(x));
-        dwr_reduce_kernel<<<ceil_div(E * d, 256), 256, 0, s>>>(b->dwr_part, b->d_router, E * d, slices);
-        dbias_kernel<<<E, 256, 0, s>>>(b->dl, b->d_bias, T, E);
-        BW_TRY(cudaGetLastError());
+        BW_TRY(x_is_compute ? run(static_cast<const CT *>(x)) : run(static_cast<const OT *>(x)));
+        BW_TRY(launch_ex(dwr_reduce_kernel, dim3(ceil_div(E * d, 256)), dim3(256), 0, s, pdl, b->dwr_part, b->d_router, E * d,
+                         slices));
+        BW_TRY(launch_ex(dbias_kernel, dim3(E), dim3(256), 0, s, pdl, b->dl, b->d_bias, T, E));
         *n += 3;
     }
     if (T > 0) {
         const EpWait wt = ep ? ep_out_wait(h) : EpWait{nullptr, 1, nullptr, 0};
-        dx_kernel<CT, OT><<<tblocks, 256, warps * E * sizeof(float), s>>>(
-            b->dxp_table, El, h->topk_idx, wt, h->dev_err, h->pos, b->dl, h->w_router, static_cast<OT *>(dx), T, d, k, E);
-        BW_TRY(cudaGetLastError());
+        BW_TRY(launch_ex(dx_kernel<CT, OT>, dim3(tblocks), dim3(256), warps * E * sizeof(float), s, pdl, b->dxp_table, El,
+                         h->topk_idx, wt, h->dev_err, h->pos, b->dl, h->w_router, static_cast<OT *>(dx), T, d, k, E));
         (*n)++;
     }
     return cudaSuccess;
@@ -668,6 +680,8 @@ __global__ void __launch_bounds__(256)
 rmsnorm_bwd_kernel(const OT *__restrict__ x, const float *__restrict__ gamma, const OT *__restrict__ dxn,
                    const OT *__restrict__ dy, OT *__restrict__ dx, float *__restrict__ inv_rms, float eps, int T,
                    int d) {
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= T) return;
@@ -704,36 +718,56 @@ rmsnorm_bwd_kernel(const OT *__restrict__ x, const float *__restrict__ gamma, co
     }
 }
 
-// d gamma[c] = sum_t (x[t,c] / rms_t) * dxn[t,c]: thread = column, blockIdx.y = slice of the tokens;
-// partials [slices][d] are added in order by dwr_reduce_kernel.
+// d gamma[c] = sum_t (x[t,c] / rms_t) * dxn[t,c]: a block takes 64 columns (two per lane) of one slice of the tokens, warp w
+// every eighth token from w on; the warps' sums are added in order, the partials [slices][d] by dwr_reduce_kernel.
 template <typename OT>
 __global__ void __launch_bounds__(256)
 dgamma_partial_kernel(const OT *__restrict__ x, const OT *__restrict__ dxn, const float *__restrict__ inv_rms,
                       float *__restrict__ part, int T, int d, int slices) {
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    if (c >= d) return;
+    __shared__ float s_sum[8][64];
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.x * 64 + lane * 2;
     const int per = (T + slices - 1) / slices;
     const int t0 = blockIdx.y * per, t1 = min(T, t0 + per);
-    float acc = 0.f;
-#pragma unroll 8
-    for (int t = t0; t < t1; t++) acc = fmaf(ldf(x + (size_t)t * d + c) * inv_rms[t], ldf(dxn + (size_t)t * d + c), acc);
-    part[(size_t)blockIdx.y * d + c] = acc;
+    float a0 = 0.f, a1 = 0.f;
+    if (c < d) {  // d is a multiple of 8: a pair of columns is whole or absent
+#pragma unroll 4
+        for (int t = t0 + warp; t < t1; t += 8) {
+            float x0, x1, g0, g1;
+            ld_pair(x + (size_t)t * d + c, x0, x1);
+            ld_pair(dxn + (size_t)t * d + c, g0, g1);
+            const float r = inv_rms[t];
+            a0 = fmaf(x0 * r, g0, a0);
+            a1 = fmaf(x1 * r, g1, a1);
+        }
+    }
+    s_sum[warp][lane * 2] = a0;
+    s_sum[warp][lane * 2 + 1] = a1;
+    __syncthreads();
+    const int col = blockIdx.x * 64 + threadIdx.x;
+    if (threadIdx.x < 64 && col < d) {
+        float acc = s_sum[0][threadIdx.x];
+#pragma unroll
+        for (int w = 1; w < 8; w++) acc += s_sum[w][threadIdx.x];
+        part[(size_t)blockIdx.y * d + col] = acc;
+    }
 }
 
 template <typename OT>
 cudaError_t block_tail_t(omoe_handle *h, BwState *b, const void *x, const float *gamma, float eps, const void *dy,
                          void *dx, float *dgamma, int T, cudaStream_t s, int *n) {
     const int d = h->cfg.d_model, slices = b->dwr_slices;
+    const bool pdl = bw_pdl(h);
+    const OT *xr = static_cast<const OT *>(x), *dxn = static_cast<const OT *>(b->dxn);
     if (T > 0)
-        rmsnorm_bwd_kernel<OT><<<ceil_div(T, 8), 256, 0, s>>>(static_cast<const OT *>(x), gamma,
-                                                             static_cast<const OT *>(b->dxn),
-                                                             static_cast<const OT *>(dy), static_cast<OT *>(dx),
-                                                             b->inv_rms, eps, T, d);
+        BW_TRY(launch_ex(rmsnorm_bwd_kernel<OT>, dim3(ceil_div(T, 8)), dim3(256), 0, s, pdl, xr, gamma, dxn,
+                         static_cast<const OT *>(dy), static_cast<OT *>(dx), b->inv_rms, eps, T, d));
     // the partial buffer of the router's weight gradient is free again by now ([slices][E][d] >= [slices][d])
-    dgamma_partial_kernel<OT><<<dim3(ceil_div(d, 256), slices), 256, 0, s>>>(
-        static_cast<const OT *>(x), static_cast<const OT *>(b->dxn), b->inv_rms, b->dwr_part, T, d, slices);
-    dwr_reduce_kernel<<<ceil_div(d, 256), 256, 0, s>>>(b->dwr_part, dgamma, d, slices);
-    BW_TRY(cudaGetLastError());
+    BW_TRY(launch_ex(dgamma_partial_kernel<OT>, dim3(ceil_div(d, 64), slices), dim3(256), 0, s, pdl, xr, dxn, b->inv_rms,
+                     b->dwr_part, T, d, slices));
+    BW_TRY(launch_ex(dwr_reduce_kernel, dim3(ceil_div(d, 256)), dim3(256), 0, s, pdl, b->dwr_part, dgamma, d, slices));
     *n += 3;
     return cudaSuccess;
 }

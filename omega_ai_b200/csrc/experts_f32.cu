@@ -237,7 +237,7 @@ template <bool B_KN, Epi EPI>
 cudaError_t launch_rows(omoe_handle *h, cudaStream_t s, const void *A, int lda, int a_next, const void *B0, const void *B1,
                         void *C, void *gu, int N, int K) {
     return launch_ex(rows_sgemm_kernel<B_KN, EPI>, dim3(ceil_div(N, BN), (unsigned)(h->rows_cap / BM)), dim3(128), 0, s,
-                     h->pdl, static_cast<const float *>(A), lda, a_next, static_cast<const float *>(B0),
+                     h->pdl && h->cfg.world == 1, static_cast<const float *>(A), lda, a_next, static_cast<const float *>(B0),
                      static_cast<const float *>(B1), static_cast<float *>(C), static_cast<float *>(gu), N, K,
                      h->ex_tile_expert, h->ex_poffsets, h->ex_counts, h->e_local);
 }
@@ -270,8 +270,8 @@ cudaError_t f32_grad_rows(omoe_handle *h, cudaStream_t s, const void *dyp, void 
 cudaError_t f32_wgrad(omoe_handle *h, cudaStream_t s, const void *a, int lda, int a_next, const void *b, int n_mat, int M,
                       int N, float *out0, float *out1) {
     const int El = h->e_local;
-    return launch_ex(wgrad_sgemm_kernel, dim3(ceil_div(N, 64), ceil_div(M, 64), n_mat * El), dim3(256), 0, s, h->pdl,
-                     static_cast<const float *>(a), lda, a_next, static_cast<const float *>(b), N, out0, out1, M, N,
+    return launch_ex(wgrad_sgemm_kernel, dim3(ceil_div(N, 64), ceil_div(M, 64), n_mat * El), dim3(256), 0, s,
+                     h->pdl && h->cfg.world == 1, static_cast<const float *>(a), lda, a_next, static_cast<const float *>(b), N, out0, out1, M, N,
                      h->ex_poffsets, h->ex_counts, El);
 }
 

@@ -77,6 +77,7 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
 
+    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStagesW; s++) {
             mbar_init(full_bar(s), 1);
@@ -95,6 +96,7 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    pdl_wait();  // everything from here on reads what earlier kernels wrote
     tc_fence_before();
     cluster_sync_all();
     tc_fence_after();
@@ -247,7 +249,7 @@ cudaError_t launch_wgrad(omoe_handle *h, cudaStream_t s, const WgradMaps &maps, 
         if (e != cudaSuccess) return e;
         if (done) *done = true;
     }
-    return launch_ex(wgrad_kernel, dim3(h->sm_count & ~1), dim3(kThreadsW), kSmemBytesW, s, false, maps, n_mat, M, N,
+    return launch_ex(wgrad_kernel, dim3(h->sm_count & ~1), dim3(kThreadsW), kSmemBytesW, s, h->pdl && h->cfg.world == 1, maps, n_mat, M, N,
                      h->ex_poffsets, h->ex_counts, h->e_local, h->dev_err);
 }
 
