@@ -16,7 +16,8 @@
 // [rows, 2*d_ff], g in the left half), h, yp and the routing.
 //
 // bf16 layers: every product runs on pairs of SMs (experts_sm100_pair.cu, experts_sm100_wgrad.cu).  The training
-// forward's up/gate product stores g and u beside h from one accumulator.  The two input-gradient products read the
+// forward's up/gate product stores g and u beside h from one accumulator.  The first product of the
+// backward turns dh into dg and du in its epilogue; it and dxp read the
 // forward's weights as they lie, as MN-major operands (dxp = dg * W_gate + du * W_up is ONE product with two sources), so
 // there are no transposed copies to refresh when the weights change: on the Mixtral-shaped layer those were 2.8 GB of
 // memory and three passes over the weights after every omoe_set_weights.  The weight-gradient products reduce over an
@@ -45,7 +46,6 @@ struct BwState {
     float *inv_rms;   // [t_max] 1/rms of every row (block form)
     void *gu;         // [rows_cap, 2*dff] g | u (compute dtype)
     void *dyp;        // [rows_cap, d]
-    void *dh;         // [rows_cap, dff]
     void *dgu;        // [rows_cap, 2*dff] dg | du
     void *dxp;        // [rows_cap, d]
     float *dgw;       // [t_max*k] gradient of the gate weights
@@ -57,42 +57,11 @@ struct BwState {
     // gradients (fp32)
     float *d_router, *d_bias, *d_gate, *d_up, *d_down;
     // tensor maps of the bf16 products
-    PairMaps up, dh_maps, dxp_maps;  // up/gate keeping g and u; dyp * W_down; dg * W_gate + du * W_up
+    PairMaps up, back, dxp_maps;  // up/gate keeping g and u; dyp * W_down and SwiGLU's backward; dg * W_gate + du * W_up
     WgradMaps w_down, w_gu;
 };
 
 namespace {
-
-__device__ __forceinline__ float silu_f32(float x) { return x / (1.0f + expf(-x)); }
-__device__ __forceinline__ float silu_grad_f32(float x) {
-    const float sg = 1.0f / (1.0f + expf(-x));
-    return sg * (1.0f + x * (1.0f - sg));
-}
-
-// ---- element-wise passes over the rows in use -----------------------------------------------------
-// dg = (dh * u) * silu'(g), du = dh * silu(g); dgu is [rows, 2*dff] with dg in the left half.
-template <typename T>
-__global__ void __launch_bounds__(256)
-swiglu_bwd_kernel(const T *__restrict__ dh, const T *__restrict__ gu, T *__restrict__ dgu,
-                  const int32_t *__restrict__ rows_in_use, int dff) {
-    pdl_trigger();
-    pdl_wait();
-    const int64_t vec = dff / 8, total = (int64_t)*rows_in_use * vec;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / vec, c = (i % vec) * 8;
-        float g[8], u[8], dv[8], dg[8], du[8];
-        load8(gu + r * 2 * dff + c, g);
-        load8(gu + r * 2 * dff + dff + c, u);
-        load8(dh + r * dff + c, dv);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            du[j] = dv[j] * silu_f32(g[j]);
-            dg[j] = (dv[j] * u[j]) * silu_grad_f32(g[j]);
-        }
-        store8(dgu + r * 2 * dff + c, dg);
-        store8(dgu + r * 2 * dff + dff + c, du);
-    }
-}
 
 // ---- combine backward + router backward: one warp per token ---------------------------------------
 // dyp[pos_j] = w_j * dy[t];  d w_j = <dy[t], yp[pos_j]>;  then lane 0 turns the k values d w into the
@@ -368,12 +337,6 @@ zero_pad_rows_kernel(__nv_bfloat16 *__restrict__ buf, int ld, const int32_t *__r
         base[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-int grid_for(int64_t work_items, int sm_count) {
-    int64_t b = (work_items + 255) / 256;
-    const int64_t cap = (int64_t)sm_count * 8;
-    return (int)(b < 1 ? 1 : (b > cap ? cap : b));
-}
-
 #define BW_TRY(expr)                                  \
     do {                                              \
         cudaError_t _e = (expr);                      \
@@ -402,7 +365,6 @@ template <typename CT, typename OT>
 cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_compute, const void *dy, void *dx, int T,
                        cudaStream_t s, int *n) {
     const int d = h->cfg.d_model, dff = h->cfg.d_ff, El = h->e_local, E = h->cfg.n_experts, k = h->cfg.top_k;
-    const int32_t *rows_in_use = h->ex_poffsets + El;
     const int warps = 8, tblocks = ceil_div(T, warps);
     const bool ep = h->cfg.world > 1, pdl = bw_pdl(h);
     EpSignal sig{nullptr, 1, 0, nullptr};
@@ -427,12 +389,8 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
         BW_TRY(launch_ex(zero_pad_rows_kernel, dim3(El, 8), dim3(256), 0, s, pdl, static_cast<CT *>(b->dyp), d, h->ex_poffsets,
                          h->ex_counts));
         (*n)++;
-        const int ew_grid = grid_for(h->rows_cap * (int64_t)dff / 8, h->sm_count);
-        // dh = dyp * W_down; rows up to a multiple of 64, because the weight gradients reduce over blocks of 64 rows
-        BW_TRY(launch_pair(h, s, pdl, PairKind::kPlainMN, b->dh_maps, dff, d, 64));
-        (*n)++;
-        BW_TRY(launch_ex(swiglu_bwd_kernel<CT>, dim3(ew_grid), dim3(256), 0, s, pdl, static_cast<const CT *>(b->dh),
-                         static_cast<const CT *>(b->gu), static_cast<CT *>(b->dgu), rows_in_use, dff));
+        // dg | du from dh = dyp * W_down; rows up to a multiple of 64, because the weight gradients reduce over blocks of 64 rows
+        BW_TRY(launch_pair(h, s, pdl, PairKind::kSwigluBack, b->back, dff, d, 64));
         (*n)++;
         BW_TRY(launch_pair(h, s, pdl, PairKind::kPlainMN2, b->dxp_maps, d, dff, 32));
         (*n)++;
@@ -483,7 +441,7 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
 
 void free_state(BwState *b) {
     if (!b->own_grad_rows) b->dyp = b->dxp = nullptr, b->dyp_table = b->dxp_table = nullptr;
-    void *ptrs[] = {b->dyp_table, b->dxp_table, b->gu, b->dyp, b->dh, b->dgu, b->dxp, b->dgw, b->dl, b->dwr_part, b->d_router, b->d_bias, b->d_gate, b->d_up, b->d_down, b->aux_ps, b->dxn, b->inv_rms};
+    void *ptrs[] = {b->dyp_table, b->dxp_table, b->gu, b->dyp, b->dgu, b->dxp, b->dgw, b->dl, b->dwr_part, b->d_router, b->d_bias, b->d_gate, b->d_up, b->d_down, b->aux_ps, b->dxn, b->inv_rms};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete b;
@@ -506,8 +464,7 @@ int bw_set_training(omoe_handle *h, int on) {
     const size_t E = h->cfg.n_experts, tm = h->cfg.t_max, k = h->cfg.top_k;
     b->dwr_slices = (int)(tm >= 4096 ? 64 : (tm >= 256 ? 8 : 1));
     struct { void **p; size_t bytes; } bufs[] = {
-        {&b->gu, rows * 2 * dff * cs}, {&b->dh, rows * dff * cs},
-        {&b->dgu, rows * 2 * dff * cs}, {(void **)&b->dgw, tm * k * 4},
+        {&b->gu, rows * 2 * dff * cs}, {&b->dgu, rows * 2 * dff * cs}, {(void **)&b->dgw, tm * k * 4},
         {(void **)&b->dl, tm * E * 4}, {(void **)&b->dwr_part, (size_t)b->dwr_slices * E * d * 4},
         {(void **)&b->d_router, E * d * 4}, {(void **)&b->d_bias, E * 4}, {(void **)&b->aux_ps, E * 4}, {(void **)&b->d_gate, El * dff * d * 4},
         {(void **)&b->d_up, El * dff * d * 4}, {(void **)&b->d_down, El * dff * d * 4}};
@@ -554,10 +511,9 @@ int bw_set_training(omoe_handle *h, int on) {
         b->up = h->maps.up;
         bool m = encode_map_bf16(&b->up.o1, gu, rows, dff, 2 * dff, 32) &&
                  encode_map_bf16(&b->up.o2, gu + dff, rows, dff, 2 * dff, 32) &&
-                 weights(&b->dh_maps.a0, h->w_down, d, dff) &&
-                 encode_map_bf16(&b->dh_maps.b0, b->dyp, rows, d, d, 128) &&
-                 encode_map_bf16(&b->dh_maps.b0_32, b->dyp, rows, d, d, 32) &&
-                 encode_map_bf16(&b->dh_maps.o0, b->dh, rows, dff, dff, 32) &&
+                 weights(&b->back.a0, h->w_down, d, dff) &&
+                 encode_map_bf16(&b->back.b0, b->dyp, rows, d, d, 128) &&
+                 encode_map_bf16(&b->back.b0_32, b->dyp, rows, d, d, 32) &&
                  weights(&b->dxp_maps.a0, h->w_gate, dff, d) && weights(&b->dxp_maps.a1, h->w_up, dff, d) &&
                  encode_map_bf16(&b->dxp_maps.b0, dgu, rows, dff, 2 * dff, 128) &&
                  encode_map_bf16(&b->dxp_maps.b0_32, dgu, rows, dff, 2 * dff, 32) &&
@@ -570,6 +526,10 @@ int bw_set_training(omoe_handle *h, int on) {
                  encode_map_bf16(&b->w_gu.a1, dgu + dff, rows, dff, 2 * dff, 64) &&
                  encode_map_bf16(&b->w_gu.b, h->xp, rows, d, d, 64) && grads(&b->w_gu.o0, b->d_gate, dff, d) &&
                  grads(&b->w_gu.o1, b->d_up, dff, d);
+        b->back.s0 = b->up.o1;  // g, u in; dg, du out
+        b->back.s1 = b->up.o2;
+        b->back.o0 = b->dxp_maps.b0_32;
+        b->back.o1 = b->dxp_maps.b1_32;
         if (!m) {
             free_state(b);
             snprintf(h->err, sizeof(h->err), "omoe_set_training: cuTensorMapEncodeTiled failed");

@@ -3,8 +3,8 @@
 //
 //   up/gate:  h  = silu(xp * Wg^T) * (xp * Wu^T)       (training: g and u are stored too)
 //   plain:    yp = h * Wd^T                            (K-major weights, as they lie)
-//   plain MN: dh = dyp * Wd                            (the same weights with the reduction along their slow index)
-//             dxp = dg * Wg + du * Wu                  (two such sources, one accumulator)
+//   back:     dg, du from dh = dyp * Wd                (the weights with the reduction along their slow index; dh stays here)
+//   plain MN: dxp = dg * Wg + du * Wu                  (two such sources, one accumulator)
 //
 // What bounds it: the tensor pipe on large steps, and on the way there the shared-memory fill (L2 -> SM).  A CTA with a
 // 128 x 256 tile of its own pulls 48 KB per 64-deep k-block; a pair shares one 256 x 256 tile, each CTA holding half of
@@ -36,17 +36,28 @@ namespace omoe {
 namespace {
 
 using namespace sm100;
-constexpr int kStagesP = 6;
 constexpr int kAccStagesP = 2;
 constexpr int kTmemColsP = 512;
 constexpr int kABytesP = 128 * BLOCK_K * 2;       // 16 KB: this CTA's half of the 256 weight rows
 constexpr int kStageBytesP = 2 * kABytesP;        // and up to 128 of the tile's (<= 256) token rows
-constexpr int kOutHalfBytesP = 16384;             // staging of one epilogue half (4 warps)
+// Ring depth and staging bytes of one epilogue half (4 warps).  Six stages and one 16 KB pass of results fit; the epilogues
+// that move three results, or two rows in and two out, per pass of 64 tokens take a stage for it (five stages instead of
+// six cost 1 % of a forward).  Against a pass over the accumulator per result and a SwiGLU kernel between the products: training step of
+// 4096 tokens, d 1024, d_ff 2816 673 -> 661 us, of 8192 tokens, d 4096, d_ff 14336 18.3 -> 17.9 ms.
+template <PairKind KIND>
+struct PairSmem {
+    static constexpr int kStages = (KIND == PairKind::kUpGateKeep || KIND == PairKind::kSwigluBack) ? 5 : 6;
+    static constexpr int kHalf = KIND == PairKind::kUpGateKeep ? 3 * 8192 : (KIND == PairKind::kSwigluBack ? 32768 : 16384);
+};
 constexpr int kTableInts = 3 * kMaxExperts + 1;   // token-tile prefix, counts, first rows of the local experts
 constexpr int kBarBytesP = 256;
-constexpr int kSmemBytesP =
-    kStagesP * kStageBytesP + 2 * kOutHalfBytesP + kBarBytesP + kTableInts * 4 + 1024 /*align slack*/;
-static_assert(kSmemBytesP <= 227 * 1024, "shared memory of one CTA");
+template <PairKind KIND>
+constexpr int pair_smem_bytes() {
+    return PairSmem<KIND>::kStages * kStageBytesP + 2 * PairSmem<KIND>::kHalf + kBarBytesP + kTableInts * 4 + 1024 /*align slack*/;
+}
+static_assert(pair_smem_bytes<PairKind::kUpGate>() <= 227 * 1024 && pair_smem_bytes<PairKind::kUpGateKeep>() <= 227 * 1024 &&
+                  pair_smem_bytes<PairKind::kSwigluBack>() <= 227 * 1024,
+              "shared memory of one CTA");
 constexpr int kThreadsP = 320;
 constexpr int kTokensMax = 256;  // token columns of a tile
 
@@ -66,7 +77,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsP, 1)
 pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const int32_t *__restrict__ poffsets,
                  const int32_t *__restrict__ counts, int E, int cap, int row_round, int kband, int32_t *dev_err) {
     constexpr bool kGate = KIND == PairKind::kUpGate || KIND == PairKind::kUpGateKeep;
-    constexpr bool kMN = KIND == PairKind::kPlainMN || KIND == PairKind::kPlainMN2;
+    constexpr bool kMN = KIND == PairKind::kSwigluBack || KIND == PairKind::kPlainMN2;
+    constexpr int kStagesP = PairSmem<KIND>::kStages, kOutHalfBytesP = PairSmem<KIND>::kHalf;
     constexpr int kFeatPair = kGate ? 128 : 256;  // output features of a pair's tile
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -79,7 +91,8 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
     auto empty_bar = [&](int s) { return bar0 + 8u * (kStagesP + s); };
     auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kStagesP + s); };
     auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStagesP + kAccStagesP + s); };
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 8 * (2 * kStagesP + 2 * kAccStagesP));
+    auto in_bar = [&](int half) { return bar0 + 8u * (2 * kStagesP + 2 * kAccStagesP + half); };  // kSwigluBack: g and u are in
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 8 * (2 * kStagesP + 2 * kAccStagesP + 2));
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     int *s_tt = reinterpret_cast<int *>(bar_ptr + kBarBytesP);  // [E+1] token tiles before each expert
     int *s_cnt = s_tt + kMaxExperts + 1, *s_row = s_cnt + kMaxExperts;
@@ -98,6 +111,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
             mbar_init(tfull_bar(s), 1);
             mbar_init(tempty_bar(s), 16);  // one arrival per epilogue warp of both CTAs
         }
+        for (int i = 0; i < 2; i++) mbar_init(in_bar(i), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -264,10 +278,40 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 : "=r"(r) : "r"((uint32_t)ok), "r"(1 + half) : "memory");
             return r != 0;
         };
-        auto put = [&](uint32_t sub, int row, int f, uint32_t word) {  // features f, f+1 (f even, < 64) of a token row
-            const uint32_t a = sub + row * 128 + ((((uint32_t)f >> 3) ^ (row & 7)) << 4) + (f & 6) * 2;
-            asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(word) : "memory");
+        auto word_at = [&](uint32_t sub, int row, int f) {  // features f, f+1 (f even, < 64) of a token row
+            return sub + row * 128 + ((((uint32_t)f >> 3) ^ (row & 7)) << 4) + (f & 6) * 2;
         };
+        auto put = [&](uint32_t sub, int row, int f, uint32_t word) {
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(word_at(sub, row, f)), "r"(word) : "memory");
+        };
+        // kSwigluBack: the issuer fetches g and u of the passes (64 tokens of this half) one ahead of the arithmetic, so the
+        // first pass of a tile is there before its accumulator is
+        int in_tile = pair0, in_p = 0;
+        uint32_t in_phase = 0;
+        bool gone = false;
+        auto request_next = [&]() {
+            int cols = 0;
+            PairTile t{};
+            for (; in_tile < total; in_tile += pairs, in_p = 0) {
+                t = tile_at(in_tile);
+                cols = min(max(t.n - half * 128, 0), 128);
+                if (in_p < cols) break;
+            }
+            if (in_tile >= total) return;
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the stores have read the staging rows
+            const int x0 = t.ft * 256 + (int)rank * 128, y0 = t.row0 + half * 128 + in_p;
+            const int subs = min(max((n_out - x0 + 63) / 64, 0), 2), top = min(64, cols - in_p);
+            mbar_expect_tx(in_bar(half), (uint32_t)(2 * subs * (top / 32) * 4096));
+            for (int q = 0; q < subs; q++)
+                for (int c = 0; c < top; c += 32) {
+                    tma_load_2d(stg + q * 8192 + c * 128, &maps.s0, in_bar(half), x0 + 64 * q, y0 + c);
+                    tma_load_2d(stg + 16384 + q * 8192 + c * 128, &maps.s1, in_bar(half), x0 + 64 * q, y0 + c);
+                }
+            in_p += 64;
+        };
+        if constexpr (KIND == PairKind::kSwigluBack) {
+            if (issuer) request_next();
+        }
         int as = 0;
         uint32_t aphase = 0;
         for (int tile = pair0; tile < total; tile += pairs) {
@@ -275,7 +319,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
             const bool ok = mbar_wait(tfull_bar(as), aphase, abort_flag, dev_err);
             __syncwarp();
             // the last stores of the tile before must have finished reading the staging rows
-            if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            if (KIND != PairKind::kSwigluBack && issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             if (!half_all(ok)) break;
             tc_fence_after();
             const int cols = min(max(t.n - half * 128, 0), 128);  // this half's token columns (a multiple of 32)
@@ -290,47 +334,114 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 const int up = (lane >> 3) & 1;  // lanes 8-15 and 24-31 hold up rows, the others gate rows
                 const int f = quarter * 16 + ((lane >> 4) << 3) + (lane & 6);
                 const int x0 = t.ft * 128 + (int)rank * 64;
-                constexpr int kOuts = KIND == PairKind::kUpGateKeep ? 3 : 1;
-#pragma unroll
-                for (int o = 0; o < kOuts; o++) {  // h, then g and u
-                    if (o > 0) {
+                constexpr int kOuts = KIND == PairKind::kUpGateKeep ? 3 : 1;  // h; with kUpGateKeep g and u too
+                constexpr int kPass = kOuts == 3 ? 64 : 128;                   // tokens staged at a time
+                for (int p = 0; p < cols; p += kPass) {
+                    if (p > 0) {
                         if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                         half_sync();
                     }
-                    for (int c = 0; c < cols; c += 32) {
+                    const int top = min(kPass, cols - p);
+                    for (int c = 0; c < top; c += 32) {
                         uint32_t r[32];
-                        tc_ld32(t_acc + c, r);
+                        tc_ld32(t_acc + p + c, r);
                         tc_wait_ld();
-                        if (o == kOuts - 1 && c + 32 >= cols) release();
-                        float v[16];
+                        if (p + c + 32 >= cols) release();
+                        float g[16], u[16];
 #pragma unroll
                         for (int i = 0; i < 16; i++) {
                             // a gate lane finishes token 2i, its up lane token 2i + 1
                             const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[2 * i] : r[2 * i + 1], 8);
-                            float g = __uint_as_float(up ? got : r[2 * i]);
-                            float u = __uint_as_float(up ? r[2 * i + 1] : got);
-                            if constexpr (KIND == PairKind::kUpGateKeep) {
+                            g[i] = __uint_as_float(up ? got : r[2 * i]);
+                            u[i] = __uint_as_float(up ? r[2 * i + 1] : got);
+                            if constexpr (kOuts == 3) {
                                 // h follows from the g and u that are kept: what the backward differentiates
-                                g = __bfloat162float(__float2bfloat16_rn(g));
-                                u = __bfloat162float(__float2bfloat16_rn(u));
+                                g[i] = __bfloat162float(__float2bfloat16_rn(g[i]));
+                                u[i] = __bfloat162float(__float2bfloat16_rn(u[i]));
                             }
-                            v[i] = o == 0 ? silu_f(g) * u : (o == 1 ? g : u);
+                        }
+                        // an even feature's lane finishes the first of two tokens, its neighbour the second
+                        auto out = [&](uint32_t dst, const float (&v)[16]) {
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
+                                put(dst, c + 4 * i + 2 * odd + up, f, odd ? pack_bf16(got, v[2 * i + 1]) : pack_bf16(v[2 * i], got));
+                            }
+                        };
+                        if constexpr (kOuts == 3) {
+                            out(stg + 8192, g);
+                            out(stg + 16384, u);
                         }
 #pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            // an even feature's lane finishes the first of two tokens, its neighbour the second
-                            const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
-                            put(stg, c + 4 * i + 2 * odd + up, f, odd ? pack_bf16(got, v[2 * i + 1]) : pack_bf16(v[2 * i], got));
-                        }
+                        for (int i = 0; i < 16; i++) g[i] = silu_f(g[i]) * u[i];
+                        out(stg, g);
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     half_sync();
                     if (issuer && x0 < n_out) {
-                        const CUtensorMap *mo = o == 0 ? &maps.o0 : (o == 1 ? &maps.o1 : &maps.o2);
-                        for (int c = 0; c < cols; c += 32) tma_store_2d(mo, stg + c * 128, x0, y0 + c);
+                        for (int c = 0; c < top; c += 32) {
+                            tma_store_2d(&maps.o0, stg + c * 128, x0, y0 + p + c);
+                            if constexpr (kOuts == 3) {
+                                tma_store_2d(&maps.o1, stg + 8192 + c * 128, x0, y0 + p + c);
+                                tma_store_2d(&maps.o2, stg + 16384 + c * 128, x0, y0 + p + c);
+                            }
+                        }
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 }
+                if (cols == 0) release();
+            } else if constexpr (KIND == PairKind::kSwigluBack) {
+                const int f = (quarter * 32 + lane) & 62;
+                const uint32_t sub = stg + (quarter >> 1) * 8192;  // g of 64 tokens x 64 features; u 16 KB on
+                const int x0 = t.ft * 256 + (int)rank * 128;
+                for (int p = 0; p < cols; p += 64) {
+                    const bool in = mbar_wait(in_bar(half), in_phase, abort_flag, dev_err);
+                    __syncwarp();
+                    if (!half_all(in)) { gone = true; break; }
+                    in_phase ^= 1u;
+                    const int top = min(64, cols - p);
+                    for (int c = 0; c < top; c += 32) {
+                        uint32_t r[32];
+                        tc_ld32(t_acc + p + c, r);
+                        tc_wait_ld();
+                        if (p + c + 32 >= cols) release();
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            const float own = __uint_as_float(odd ? r[2 * i + 1] : r[2 * i]);
+                            const float got = __uint_as_float(__shfl_xor_sync(0xffffffffu, odd ? r[2 * i] : r[2 * i + 1], 1));
+                            // dh in the layer's element type, as a pass of its own would read it
+                            const uint32_t dh = odd ? pack_bf16(got, own) : pack_bf16(own, got);
+                            const uint32_t a = word_at(sub, c + 2 * i + odd, f);
+                            uint32_t g, u;
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(g) : "r"(a) : "memory");
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(u) : "r"(a + 16384) : "memory");
+                            float dg[2], du[2];
+#pragma unroll
+                            for (int q = 0; q < 2; q++) {
+                                auto half_of = [&](uint32_t w) { return __uint_as_float(q ? w & 0xffff0000u : w << 16); };
+                                const float x = half_of(g), d = half_of(dh);
+                                const float sg = __fdividef(1.0f, 1.0f + __expf(-x));
+                                du[q] = d * (x * sg);
+                                dg[q] = (d * half_of(u)) * (sg * (1.0f + x * (1.0f - sg)));
+                            }
+                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(pack_bf16(dg[0], dg[1])) : "memory");
+                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + 16384), "r"(pack_bf16(du[0], du[1])) : "memory");
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    half_sync();
+                    if (issuer) {
+                        for (int c = 0; c < top; c += 32)
+                            for (int q = 0; q < 2; q++)
+                                if (x0 + 64 * q < n_out) {
+                                    tma_store_2d(&maps.o0, stg + q * 8192 + c * 128, x0 + 64 * q, y0 + p + c);
+                                    tma_store_2d(&maps.o1, stg + 16384 + q * 8192 + c * 128, x0 + 64 * q, y0 + p + c);
+                                }
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        request_next();
+                    }
+                }
+                if (gone) break;
                 if (cols == 0) release();
             } else {
                 const int f = (quarter * 32 + lane) & 62;
@@ -369,6 +480,10 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
             if (++as == kAccStagesP) { as = 0; aphase ^= 1u; }
         }
         if (issuer) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (*abort_flag && KIND == PairKind::kSwigluBack) {
+            const unsigned long long t0 = globaltimer_ns();  // let g and u that were already requested land
+            while (globaltimer_ns() - t0 < 2000000ull) { }
+        }
     }
 
     tc_fence_before();
@@ -384,11 +499,12 @@ cudaError_t launch_pair_t(omoe_handle *h, cudaStream_t s, bool pdl, const PairMa
     static PerDeviceOnce once;  // one per instantiation
     bool *done = once.slot();
     if (!done || !*done) {
-        cudaError_t e = cudaFuncSetAttribute(pair_gemm_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytesP);
+        cudaError_t e = cudaFuncSetAttribute(pair_gemm_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             pair_smem_bytes<KIND>());
         if (e != cudaSuccess) return e;
         if (done) *done = true;
     }
-    return launch_ex(pair_gemm_kernel<KIND>, dim3(h->sm_count & ~1), dim3(kThreadsP), kSmemBytesP, s, pdl, maps, n_out, K,
+    return launch_ex(pair_gemm_kernel<KIND>, dim3(h->sm_count & ~1), dim3(kThreadsP), pair_smem_bytes<KIND>(), s, pdl, maps, n_out, K,
                      h->ex_poffsets, h->ex_counts, h->e_local, kTokensMax, row_round, 8, h->dev_err);
 }
 
@@ -400,7 +516,7 @@ cudaError_t launch_pair(omoe_handle *h, cudaStream_t s, bool pdl, PairKind kind,
         case PairKind::kUpGate: return launch_pair_t<PairKind::kUpGate>(h, s, pdl, maps, n_out, K, row_round);
         case PairKind::kUpGateKeep: return launch_pair_t<PairKind::kUpGateKeep>(h, s, pdl, maps, n_out, K, row_round);
         case PairKind::kPlain: return launch_pair_t<PairKind::kPlain>(h, s, pdl, maps, n_out, K, row_round);
-        case PairKind::kPlainMN: return launch_pair_t<PairKind::kPlainMN>(h, s, pdl, maps, n_out, K, row_round);
+        case PairKind::kSwigluBack: return launch_pair_t<PairKind::kSwigluBack>(h, s, pdl, maps, n_out, K, row_round);
         case PairKind::kPlainMN2: return launch_pair_t<PairKind::kPlainMN2>(h, s, pdl, maps, n_out, K, row_round);
     }
     return cudaErrorInvalidValue;
