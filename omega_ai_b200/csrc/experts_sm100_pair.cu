@@ -23,7 +23,7 @@
 // together, one more packs neighbouring features into a word, and the rows leave through swizzled staging and
 // TMA stores of 32-token boxes.
 //
-// Roles per CTA: warp 0 producer (TMA), warp 1 of the even CTA issues the MMAs for both, warps 2-9 epilogue.  A load
+// Roles per CTA: warp 0 producer (TMA), warp 1 of the even CTA issues the MMAs for both, the others epilogue.  A load
 // signals the even CTA's "full" barrier; commits free the stage in both CTAs.  All mbarrier waits are bounded
 // (sm100_ptx.cuh): when one runs out the kernel raises the device error word, lets outstanding copies land and leaves;
 // the cluster barriers are reached by every thread whatever happened before.
@@ -40,25 +40,34 @@ constexpr int kAccStagesP = 2;
 constexpr int kTmemColsP = 512;
 constexpr int kABytesP = 128 * BLOCK_K * 2;       // 16 KB: this CTA's half of the 256 weight rows
 constexpr int kStageBytesP = 2 * kABytesP;        // and up to 128 of the tile's (<= 256) token rows
-// Ring depth and staging bytes of one epilogue half (4 warps).  Six stages and one 16 KB pass of results fit; the epilogues
-// that move three results, or two rows in and two out, per pass of 64 tokens take a stage for it (five stages instead of
-// six cost 1 % of a forward).  Against a pass over the accumulator per result and a SwiGLU kernel between the products: training step of
-// 4096 tokens, d 1024, d_ff 2816 673 -> 661 us, of 8192 tokens, d 4096, d_ff 14336 18.3 -> 17.9 ms.
+// Ring depth and epilogue of a kind.  The epilogue is kParts groups of four warps, each with 256 / kParts of a tile's token
+// columns, kPass of them staged at a time.  Six stages and 2 x 16 KB of results fit; the epilogues that move three
+// results, or two rows in and two out, take a stage for their staging (five stages instead of six cost 1 % of a forward) and have
+// twice the warps: with eight, shared-memory words, exponentials and arithmetic of a pass follow one another and a tile's
+// epilogue outlasts a reduction of 1024.  Sixteen gain nothing for the other two.  Against a pass over the
+// accumulator per result and a SwiGLU kernel between the products: training step of
+// 4096 tokens, d 1024, d_ff 2816 673 -> 661 us, with the second eight warps 640 us; of 8192 tokens, d 4096, d_ff 14336
+// 18.3 -> 17.9 ms.
 template <PairKind KIND>
-struct PairSmem {
-    static constexpr int kStages = (KIND == PairKind::kUpGateKeep || KIND == PairKind::kSwigluBack) ? 5 : 6;
-    static constexpr int kHalf = KIND == PairKind::kUpGateKeep ? 3 * 8192 : (KIND == PairKind::kSwigluBack ? 32768 : 16384);
+struct PairCfg {
+    static constexpr bool kWide = KIND == PairKind::kUpGateKeep || KIND == PairKind::kSwigluBack;
+    static constexpr int kStages = kWide ? 5 : 6;
+    static constexpr int kParts = kWide ? 4 : 2;
+    static constexpr int kPass = kWide ? 32 : (KIND == PairKind::kUpGate ? 128 : 64);
+    // 128-byte rows (64 features of a token) staged per token: h; h, g, u; g, u of two feature halves; two feature halves
+    static constexpr int kRows = KIND == PairKind::kUpGate ? 1 : (KIND == PairKind::kUpGateKeep ? 3 : (KIND == PairKind::kSwigluBack ? 4 : 2));
+    static constexpr int kPartBytes = kPass * kRows * 128;
+    static constexpr int kThreads = 64 + kParts * 128;
 };
 constexpr int kTableInts = 3 * kMaxExperts + 1;   // token-tile prefix, counts, first rows of the local experts
 constexpr int kBarBytesP = 256;
 template <PairKind KIND>
 constexpr int pair_smem_bytes() {
-    return PairSmem<KIND>::kStages * kStageBytesP + 2 * PairSmem<KIND>::kHalf + kBarBytesP + kTableInts * 4 + 1024 /*align slack*/;
+    return PairCfg<KIND>::kStages * kStageBytesP + PairCfg<KIND>::kParts * PairCfg<KIND>::kPartBytes + kBarBytesP + kTableInts * 4 + 1024 /*align slack*/;
 }
 static_assert(pair_smem_bytes<PairKind::kUpGate>() <= 227 * 1024 && pair_smem_bytes<PairKind::kUpGateKeep>() <= 227 * 1024 &&
                   pair_smem_bytes<PairKind::kSwigluBack>() <= 227 * 1024,
               "shared memory of one CTA");
-constexpr int kThreadsP = 320;
 constexpr int kTokensMax = 256;  // token columns of a tile
 
 // Tokens of one tile of an expert with `cnt` rows when tiles hold at most `cap` (a multiple of 32): the expert's
@@ -73,26 +82,27 @@ struct PairTile {
 };
 
 template <PairKind KIND>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsP, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<KIND>::kThreads, 1)
 pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const int32_t *__restrict__ poffsets,
                  const int32_t *__restrict__ counts, int E, int cap, int row_round, int kband, int32_t *dev_err) {
     constexpr bool kGate = KIND == PairKind::kUpGate || KIND == PairKind::kUpGateKeep;
     constexpr bool kMN = KIND == PairKind::kSwigluBack || KIND == PairKind::kPlainMN2;
-    constexpr int kStagesP = PairSmem<KIND>::kStages, kOutHalfBytesP = PairSmem<KIND>::kHalf;
+    constexpr int kStagesP = PairCfg<KIND>::kStages, kParts = PairCfg<KIND>::kParts, kPass = PairCfg<KIND>::kPass;
+    constexpr int kPartBytes = PairCfg<KIND>::kPartBytes, kPartCols = kTokensMax / kParts;
     constexpr int kFeatPair = kGate ? 128 : 256;  // output features of a pair's tile
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzled tiles start on 1024 bytes; the same in both CTAs
     unsigned char *base_ptr = smem_raw + (base - raw);
     const uint32_t out_stage = base + kStagesP * kStageBytesP;
-    const uint32_t bar0 = out_stage + 2 * kOutHalfBytesP;
-    unsigned char *bar_ptr = base_ptr + kStagesP * kStageBytesP + 2 * kOutHalfBytesP;
+    const uint32_t bar0 = out_stage + kParts * kPartBytes;
+    unsigned char *bar_ptr = base_ptr + kStagesP * kStageBytesP + kParts * kPartBytes;
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (kStagesP + s); };
     auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kStagesP + s); };
     auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStagesP + kAccStagesP + s); };
-    auto in_bar = [&](int half) { return bar0 + 8u * (2 * kStagesP + 2 * kAccStagesP + half); };  // kSwigluBack: g and u are in
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 8 * (2 * kStagesP + 2 * kAccStagesP + 2));
+    auto in_bar = [&](int part) { return bar0 + 8u * (2 * kStagesP + 2 * kAccStagesP + part); };  // kSwigluBack: g and u are in
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 8 * (2 * kStagesP + 2 * kAccStagesP + kParts));
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     int *s_tt = reinterpret_cast<int *>(bar_ptr + kBarBytesP);  // [E+1] token tiles before each expert
     int *s_cnt = s_tt + kMaxExperts + 1, *s_row = s_cnt + kMaxExperts;
@@ -109,9 +119,9 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
         }
         for (int s = 0; s < kAccStagesP; s++) {
             mbar_init(tfull_bar(s), 1);
-            mbar_init(tempty_bar(s), 16);  // one arrival per epilogue warp of both CTAs
+            mbar_init(tempty_bar(s), 8 * kParts);  // one arrival per epilogue warp of both CTAs
         }
-        for (int i = 0; i < 2; i++) mbar_init(in_bar(i), 1);
+        for (int i = 0; i < kParts; i++) mbar_init(in_bar(i), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -262,20 +272,20 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
         }
     } else {
         // ---------------- epilogue: TMEM -> registers -> shared -> TMA store ----------------
-        // warp%4 selects the 32 tensor-memory lanes (features), (warp-2)/4 the half of the token columns.  The four
-        // warps of a half share its staging and a named barrier.
-        const int ew = warp - 2, quarter = warp & 3, half = ew >> 2;
-        const uint32_t stg = out_stage + half * kOutHalfBytesP;
+        // warp%4 selects the 32 tensor-memory lanes (features), (warp-2)/4 the group, i.e. its share of
+        // the token columns.  The four warps of a group share its staging and a named barrier.
+        const int ew = warp - 2, quarter = warp & 3, part = ew >> 2;
+        const uint32_t stg = out_stage + part * kPartBytes;
         const bool issuer = (ew & 3) == 0 && lane == 0;
         const int odd = lane & 1;
-        auto half_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); };
-        // true on all 128 threads of the half or on none: its warps leave the loop together
-        auto half_all = [&](bool ok) {
+        auto part_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory"); };
+        // true on all 128 threads of the group or on none: its warps leave the loop together
+        auto part_all = [&](bool ok) {
             uint32_t r;
             asm volatile(
                 "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
                 "bar.red.and.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                : "=r"(r) : "r"((uint32_t)ok), "r"(1 + half) : "memory");
+                : "=r"(r) : "r"((uint32_t)ok), "r"(1 + part) : "memory");
             return r != 0;
         };
         auto word_at = [&](uint32_t sub, int row, int f) {  // features f, f+1 (f even, < 64) of a token row
@@ -284,7 +294,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
         auto put = [&](uint32_t sub, int row, int f, uint32_t word) {
             asm volatile("st.shared.b32 [%0], %1;" ::"r"(word_at(sub, row, f)), "r"(word) : "memory");
         };
-        // kSwigluBack: the issuer fetches g and u of the passes (64 tokens of this half) one ahead of the arithmetic, so the
+        // kSwigluBack: the issuer fetches g and u of the passes (kPass tokens of this group) one ahead of the arithmetic, so the
         // first pass of a tile is there before its accumulator is
         int in_tile = pair0, in_p = 0;
         uint32_t in_phase = 0;
@@ -294,20 +304,20 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
             PairTile t{};
             for (; in_tile < total; in_tile += pairs, in_p = 0) {
                 t = tile_at(in_tile);
-                cols = min(max(t.n - half * 128, 0), 128);
+                cols = min(max(t.n - part * kPartCols, 0), kPartCols);
                 if (in_p < cols) break;
             }
             if (in_tile >= total) return;
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the stores have read the staging rows
-            const int x0 = t.ft * 256 + (int)rank * 128, y0 = t.row0 + half * 128 + in_p;
-            const int subs = min(max((n_out - x0 + 63) / 64, 0), 2), top = min(64, cols - in_p);
-            mbar_expect_tx(in_bar(half), (uint32_t)(2 * subs * (top / 32) * 4096));
+            const int x0 = t.ft * 256 + (int)rank * 128, y0 = t.row0 + part * kPartCols + in_p;
+            const int subs = min(max((n_out - x0 + 63) / 64, 0), 2), top = min(kPass, cols - in_p);
+            mbar_expect_tx(in_bar(part), (uint32_t)(2 * subs * (top / 32) * 4096));
             for (int q = 0; q < subs; q++)
                 for (int c = 0; c < top; c += 32) {
-                    tma_load_2d(stg + q * 8192 + c * 128, &maps.s0, in_bar(half), x0 + 64 * q, y0 + c);
-                    tma_load_2d(stg + 16384 + q * 8192 + c * 128, &maps.s1, in_bar(half), x0 + 64 * q, y0 + c);
+                    tma_load_2d(stg + q * kPass * 128 + c * 128, &maps.s0, in_bar(part), x0 + 64 * q, y0 + c);
+                    tma_load_2d(stg + (2 + q) * kPass * 128 + c * 128, &maps.s1, in_bar(part), x0 + 64 * q, y0 + c);
                 }
-            in_p += 64;
+            in_p += kPass;
         };
         if constexpr (KIND == PairKind::kSwigluBack) {
             if (issuer) request_next();
@@ -320,11 +330,11 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
             __syncwarp();
             // the last stores of the tile before must have finished reading the staging rows
             if (KIND != PairKind::kSwigluBack && issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            if (!half_all(ok)) break;
+            if (!part_all(ok)) break;
             tc_fence_after();
-            const int cols = min(max(t.n - half * 128, 0), 128);  // this half's token columns (a multiple of 32)
-            const int y0 = t.row0 + half * 128;
-            const uint32_t t_acc = tmem_base + as * kTokensMax + half * 128 + ((uint32_t)(quarter * 32) << 16);
+            const int cols = min(max(t.n - part * kPartCols, 0), kPartCols);  // this group's token columns (a multiple of 32)
+            const int y0 = t.row0 + part * kPartCols;
+            const uint32_t t_acc = tmem_base + as * kTokensMax + part * kPartCols + ((uint32_t)(quarter * 32) << 16);
             auto release = [&]() {  // all of this warp's accumulator reads are done
                 tc_fence_before();
                 __syncwarp();
@@ -335,11 +345,10 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 const int f = quarter * 16 + ((lane >> 4) << 3) + (lane & 6);
                 const int x0 = t.ft * 128 + (int)rank * 64;
                 constexpr int kOuts = KIND == PairKind::kUpGateKeep ? 3 : 1;  // h; with kUpGateKeep g and u too
-                constexpr int kPass = kOuts == 3 ? 64 : 128;                   // tokens staged at a time
                 for (int p = 0; p < cols; p += kPass) {
                     if (p > 0) {
                         if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                        half_sync();
+                        part_sync();
                     }
                     const int top = min(kPass, cols - p);
                     for (int c = 0; c < top; c += 32) {
@@ -369,21 +378,21 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                             }
                         };
                         if constexpr (kOuts == 3) {
-                            out(stg + 8192, g);
-                            out(stg + 16384, u);
+                            out(stg + kPass * 128, g);
+                            out(stg + 2 * kPass * 128, u);
                         }
 #pragma unroll
                         for (int i = 0; i < 16; i++) g[i] = silu_f(g[i]) * u[i];
                         out(stg, g);
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    half_sync();
+                    part_sync();
                     if (issuer && x0 < n_out) {
                         for (int c = 0; c < top; c += 32) {
                             tma_store_2d(&maps.o0, stg + c * 128, x0, y0 + p + c);
                             if constexpr (kOuts == 3) {
-                                tma_store_2d(&maps.o1, stg + 8192 + c * 128, x0, y0 + p + c);
-                                tma_store_2d(&maps.o2, stg + 16384 + c * 128, x0, y0 + p + c);
+                                tma_store_2d(&maps.o1, stg + (kPass + c) * 128, x0, y0 + p + c);
+                                tma_store_2d(&maps.o2, stg + (2 * kPass + c) * 128, x0, y0 + p + c);
                             }
                         }
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -392,14 +401,15 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 if (cols == 0) release();
             } else if constexpr (KIND == PairKind::kSwigluBack) {
                 const int f = (quarter * 32 + lane) & 62;
-                const uint32_t sub = stg + (quarter >> 1) * 8192;  // g of 64 tokens x 64 features; u 16 KB on
+                const uint32_t sub = stg + (quarter >> 1) * kPass * 128;  // g of kPass tokens x 64 features
+                constexpr uint32_t kToU = 2 * kPass * 128;                  // u lies behind both feature halves of g
                 const int x0 = t.ft * 256 + (int)rank * 128;
-                for (int p = 0; p < cols; p += 64) {
-                    const bool in = mbar_wait(in_bar(half), in_phase, abort_flag, dev_err);
+                for (int p = 0; p < cols; p += kPass) {
+                    const bool in = mbar_wait(in_bar(part), in_phase, abort_flag, dev_err);
                     __syncwarp();
-                    if (!half_all(in)) { gone = true; break; }
+                    if (!part_all(in)) { gone = true; break; }
                     in_phase ^= 1u;
-                    const int top = min(64, cols - p);
+                    const int top = min(kPass, cols - p);
                     for (int c = 0; c < top; c += 32) {
                         uint32_t r[32];
                         tc_ld32(t_acc + p + c, r);
@@ -414,7 +424,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                             const uint32_t a = word_at(sub, c + 2 * i + odd, f);
                             uint32_t g, u;
                             asm volatile("ld.shared.b32 %0, [%1];" : "=r"(g) : "r"(a) : "memory");
-                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(u) : "r"(a + 16384) : "memory");
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(u) : "r"(a + kToU) : "memory");
                             float dg[2], du[2];
 #pragma unroll
                             for (int q = 0; q < 2; q++) {
@@ -425,17 +435,17 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                                 dg[q] = (d * half_of(u)) * (sg * (1.0f + x * (1.0f - sg)));
                             }
                             asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(pack_bf16(dg[0], dg[1])) : "memory");
-                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + 16384), "r"(pack_bf16(du[0], du[1])) : "memory");
+                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(a + kToU), "r"(pack_bf16(du[0], du[1])) : "memory");
                         }
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    half_sync();
+                    part_sync();
                     if (issuer) {
                         for (int c = 0; c < top; c += 32)
                             for (int q = 0; q < 2; q++)
                                 if (x0 + 64 * q < n_out) {
-                                    tma_store_2d(&maps.o0, stg + q * 8192 + c * 128, x0 + 64 * q, y0 + p + c);
-                                    tma_store_2d(&maps.o1, stg + 16384 + q * 8192 + c * 128, x0 + 64 * q, y0 + p + c);
+                                    tma_store_2d(&maps.o0, stg + (q * kPass + c) * 128, x0 + 64 * q, y0 + p + c);
+                                    tma_store_2d(&maps.o1, stg + kToU + (q * kPass + c) * 128, x0 + 64 * q, y0 + p + c);
                                 }
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                         request_next();
@@ -445,14 +455,14 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 if (cols == 0) release();
             } else {
                 const int f = (quarter * 32 + lane) & 62;
-                const uint32_t sub = stg + (quarter >> 1) * 8192;  // 64 tokens x 64 features
+                const uint32_t sub = stg + (quarter >> 1) * kPass * 128;  // kPass tokens x 64 features
                 const int x0 = t.ft * 256 + (int)rank * 128;
-                for (int p = 0; p < cols; p += 64) {
+                for (int p = 0; p < cols; p += kPass) {
                     if (p > 0) {
                         if (issuer) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                        half_sync();
+                        part_sync();
                     }
-                    const int top = min(64, cols - p);
+                    const int top = min(kPass, cols - p);
                     for (int c = 0; c < top; c += 32) {
                         uint32_t r[32];
                         tc_ld32(t_acc + p + c, r);
@@ -466,11 +476,11 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                         }
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    half_sync();
+                    part_sync();
                     if (issuer) {
                         for (int c = 0; c < top; c += 32) {
                             if (x0 < n_out) tma_store_2d(&maps.o0, stg + c * 128, x0, y0 + p + c);
-                            if (x0 + 64 < n_out) tma_store_2d(&maps.o0, stg + 8192 + c * 128, x0 + 64, y0 + p + c);
+                            if (x0 + 64 < n_out) tma_store_2d(&maps.o0, stg + (kPass + c) * 128, x0 + 64, y0 + p + c);
                         }
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
@@ -504,7 +514,7 @@ cudaError_t launch_pair_t(omoe_handle *h, cudaStream_t s, bool pdl, const PairMa
         if (e != cudaSuccess) return e;
         if (done) *done = true;
     }
-    return launch_ex(pair_gemm_kernel<KIND>, dim3(h->sm_count & ~1), dim3(kThreadsP), pair_smem_bytes<KIND>(), s, pdl, maps, n_out, K,
+    return launch_ex(pair_gemm_kernel<KIND>, dim3(h->sm_count & ~1), dim3(PairCfg<KIND>::kThreads), pair_smem_bytes<KIND>(), s, pdl, maps, n_out, K,
                      h->ex_poffsets, h->ex_counts, h->e_local, kTokensMax, row_round, 8, h->dev_err);
 }
 
