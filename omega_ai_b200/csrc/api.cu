@@ -398,7 +398,7 @@ static int forward_impl(omoe_handle *h, const void *x_dev, int x_dtype, void *y_
     } else {
         CU_TRY(h, launch_router(h, x_dev, x_dtype, T, s, &n));
         MARK(1);
-        CU_TRY(h, launch_scan(h, T, s, &n));
+        if (!permute_scans(h, T)) CU_TRY(h, launch_scan(h, T, s, &n));
         MARK(2);
         CU_TRY(h, launch_permute(h, x_dev, x_dtype, T, s, &n, nullptr));
     }

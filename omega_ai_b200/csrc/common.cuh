@@ -155,6 +155,8 @@ namespace omoe {
 
 cudaError_t launch_router(omoe_handle *h, const void *x, int io_dtype, int T, cudaStream_t s, int *n);
 cudaError_t launch_scan(omoe_handle *h, int T, cudaStream_t s, int *n);
+// true when launch_permute without a signal does the scan's work itself (asked after launch_router, which sets the granularity)
+bool permute_scans(const omoe_handle *h, int T);
 // Router + scan + dispatch in one launch for T <= route_small_max_tokens() (single GPU, bf16 layer).
 cudaError_t launch_route_small(omoe_handle *h, const void *x, int io_dtype, int T, cudaStream_t s, int *n);
 int route_small_max_tokens();
