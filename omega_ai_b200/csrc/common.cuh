@@ -192,6 +192,8 @@ int splitk_ways_up_gate(omoe_handle *h, long m_tiles_ub);
 // true when launch_experts_bf16 with this row bound runs the up/gate product on the persistent kernel (the one
 // that can carry the remote half of the dispatch)
 bool experts_up_is_persistent(omoe_handle *h, long rows_ub);
+// true when launch_experts_bf16 with this row bound runs either product with K split
+bool experts_split_k(omoe_handle *h, long rows_ub);
 int splitk_ways_down(omoe_handle *h, long m_tiles_ub);
 cudaError_t launch_up_gate_splitk(omoe_handle *h, cudaStream_t s, int S, const EpGate *gate);
 cudaError_t launch_down_splitk(omoe_handle *h, cudaStream_t s, int S, const EpGate *gate);

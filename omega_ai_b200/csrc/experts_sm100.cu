@@ -477,6 +477,11 @@ bool experts_up_is_persistent(omoe_handle *h, long rows_ub) {
     return splitk_ways_up_gate(h, m_tiles_bound(h, rows_ub)) == 0;
 }
 
+bool experts_split_k(omoe_handle *h, long rows_ub) {
+    const long m = m_tiles_bound(h, rows_ub);
+    return splitk_ways_up_gate(h, m) > 0 || splitk_ways_down(h, m) > 0;
+}
+
 cudaError_t launch_experts_bf16(omoe_handle *h, cudaStream_t s, int *n, cudaEvent_t mid, long rows_ub,
                                 const EpGate *gate) {
     // the up/gate product takes the wait side of the gate, the down product the signal side
