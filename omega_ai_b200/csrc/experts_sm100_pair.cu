@@ -59,12 +59,17 @@ struct PairCfg {
     static constexpr int kPartBytes = kPass * kRows * 128;
     static constexpr int kThreads = 64 + kParts * 128;
 };
-constexpr int kTableInts = 3 * kMaxExperts + 1;   // token-tile prefix, counts, first rows of the local experts
+constexpr int kTableInts = 3 * kMaxExperts + 2;   // token-tile prefix, counts, first rows of the local experts; narrow step
 constexpr int kBarBytesP = 256;
+// A step whose experts hold at most 64 rows each is bound by the weights' way from HBM: its stages need room for 32 token rows per
+// CTA, not 128, and nine of those take the ring's place (64 tokens, d 4096, d_ff 14336, 8 experts: 494 -> 479 us; 8 tokens, d 2048,
+// 64 experts: 124.3 -> 122.1 us.  Requesting the two halves of a weight row's 256 bytes together instead: 3 % slower.)
+constexpr int kStagesNarrow = 9, kStageBytesNarrow = kABytesP + 4096;
 template <PairKind KIND>
 constexpr int pair_smem_bytes() {
     return PairCfg<KIND>::kStages * kStageBytesP + PairCfg<KIND>::kParts * PairCfg<KIND>::kPartBytes + kBarBytesP + kTableInts * 4 + 1024 /*align slack*/;
 }
+static_assert(kStagesNarrow * kStageBytesNarrow <= 6 * kStageBytesP, "the narrow ring lies in the wide one's place");
 static_assert(pair_smem_bytes<PairKind::kUpGate>() <= 227 * 1024 && pair_smem_bytes<PairKind::kUpGateKeep>() <= 227 * 1024 &&
                   pair_smem_bytes<PairKind::kSwigluBack>() <= 227 * 1024,
               "shared memory of one CTA");
@@ -87,25 +92,25 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                  const int32_t *__restrict__ counts, int E, int cap, int row_round, int kband, int32_t *dev_err) {
     constexpr bool kGate = KIND == PairKind::kUpGate || KIND == PairKind::kUpGateKeep;
     constexpr bool kMN = KIND == PairKind::kSwigluBack || KIND == PairKind::kPlainMN2;
-    constexpr int kStagesP = PairCfg<KIND>::kStages, kParts = PairCfg<KIND>::kParts, kPass = PairCfg<KIND>::kPass;
+    constexpr int kRingStages = PairCfg<KIND>::kStages, kStagesMax = kRingStages == 6 ? kStagesNarrow : kRingStages, kParts = PairCfg<KIND>::kParts, kPass = PairCfg<KIND>::kPass;
     constexpr int kPartBytes = PairCfg<KIND>::kPartBytes, kPartCols = kTokensMax / kParts;
     constexpr int kFeatPair = kGate ? 128 : 256;  // output features of a pair's tile
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzled tiles start on 1024 bytes; the same in both CTAs
     unsigned char *base_ptr = smem_raw + (base - raw);
-    const uint32_t out_stage = base + kStagesP * kStageBytesP;
+    const uint32_t out_stage = base + kRingStages * kStageBytesP;
     const uint32_t bar0 = out_stage + kParts * kPartBytes;
-    unsigned char *bar_ptr = base_ptr + kStagesP * kStageBytesP + kParts * kPartBytes;
+    unsigned char *bar_ptr = base_ptr + kRingStages * kStageBytesP + kParts * kPartBytes;
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
-    auto empty_bar = [&](int s) { return bar0 + 8u * (kStagesP + s); };
-    auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kStagesP + s); };
-    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStagesP + kAccStagesP + s); };
-    auto in_bar = [&](int part) { return bar0 + 8u * (2 * kStagesP + 2 * kAccStagesP + part); };  // kSwigluBack: g and u are in
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 8 * (2 * kStagesP + 2 * kAccStagesP + kParts));
+    auto empty_bar = [&](int s) { return bar0 + 8u * (kStagesMax + s); };
+    auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kStagesMax + s); };
+    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStagesMax + kAccStagesP + s); };
+    auto in_bar = [&](int part) { return bar0 + 8u * (2 * kStagesMax + 2 * kAccStagesP + part); };  // kSwigluBack: g and u are in
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 8 * (2 * kStagesMax + 2 * kAccStagesP + kParts));
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     int *s_tt = reinterpret_cast<int *>(bar_ptr + kBarBytesP);  // [E+1] token tiles before each expert
-    int *s_cnt = s_tt + kMaxExperts + 1, *s_row = s_cnt + kMaxExperts;
+    int *s_cnt = s_tt + kMaxExperts + 1, *s_row = s_cnt + kMaxExperts, *s_narrow = s_row + kMaxExperts;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t rank;
@@ -113,7 +118,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
 
     pdl_trigger();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStagesP; s++) {
+        for (int s = 0; s < kStagesMax; s++) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -133,10 +138,11 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
     // barriers and tensor memory are set up; everything from here on reads what earlier kernels wrote
     pdl_wait();
     if (warp == 2) {
-        int run = 0;
+        int run = 0, most = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             const int cnt = e < E ? counts[e] : 0;
+            most = max(most, cnt);
             int n = (cnt + cap - 1) / cap;
             const int own = n;
 #pragma unroll
@@ -151,13 +157,19 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
             }
             run += __shfl_sync(0xffffffffu, n, 31);
         }
-        if (lane == 0) s_tt[E] = run;
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) {
+            s_tt[E] = run;
+            *s_narrow = most <= 64;
+        }
     }
     tc_fence_before();
     cluster_sync_all();  // both CTAs' barriers and tables are in place
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    const bool narrow = kRingStages == 6 && *s_narrow != 0;
+    const int kStagesP = narrow ? kStagesNarrow : kRingStages, stage_bytes = narrow ? kStageBytesNarrow : kStageBytesP;
     const int token_tiles = s_tt[E];
     const int n_ft = (n_out + kFeatPair - 1) / kFeatPair;
     const int total = token_tiles * n_ft;
@@ -204,7 +216,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 for (int kb = 0; kb < num_kb; kb++) {
                     if (!warp_wait(empty_bar(stage), phase ^ 1u, abort_flag, dev_err)) { ok = false; break; }
                     if (elect_one()) {
-                        const uint32_t sa = base + stage * kStageBytesP, sb = sa + kABytesP;
+                        const uint32_t sa = base + stage * stage_bytes, sb = sa + kABytesP;
                         const uint32_t bar = map_to_rank(full_bar(stage), 0);
                         if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * bytes);
                         const bool second = KIND == PairKind::kPlainMN2 && kb >= kb_src;
@@ -252,7 +264,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                 for (int kb = 0; kb < num_kb; kb++) {
                     if (!warp_wait(full_bar(stage), phase, abort_flag, dev_err)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t sa = base + stage * kStageBytesP;
+                    const uint32_t sa = base + stage * stage_bytes;
                     const uint64_t adesc = kMN ? make_mn_desc(sa) : make_sw128_desc(sa);
                     const uint64_t bdesc = make_sw128_desc(sa + kABytesP);
                     if (elect_one()) {
