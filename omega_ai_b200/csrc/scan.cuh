@@ -23,13 +23,20 @@ __device__ __forceinline__ void scan_body(const int32_t *__restrict__ block_coun
         int32_t *out = block_base + (size_t)e * n_blocks;
         int run = 0;
         if ((n_blocks & 3) == 0) {
-            // four blocks per lane and step (16-byte loads and stores): a quarter of the dependent round trips
-            // to L2, which are all this kernel's time
-#pragma unroll 2
-            for (int b0 = 0; b0 < n_blocks; b0 += 128) {
-                const int b = b0 + lane * 4;
-                int4 c4 = make_int4(0, 0, 0, 0);
-                if (b < n_blocks) c4 = *reinterpret_cast<const int4 *>(row + b);
+            // four blocks per lane and step (16-byte loads and stores) and the loads of eight steps together: the round
+            // trips to L2 are all this kernel's time
+            for (int b8 = 0; b8 < n_blocks; b8 += 8 * 128) {
+            int4 ahead[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int b = b8 + u * 128 + lane * 4;
+                ahead[u] = b < n_blocks ? *reinterpret_cast<const int4 *>(row + b) : make_int4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (b8 + u * 128 >= n_blocks) break;
+                const int b = b8 + u * 128 + lane * 4;
+                const int4 c4 = ahead[u];
                 const int sum4 = c4.x + c4.y + c4.z + c4.w;
                 int inc = sum4;
 #pragma unroll
@@ -42,6 +49,7 @@ __device__ __forceinline__ void scan_body(const int32_t *__restrict__ block_coun
                     *reinterpret_cast<int4 *>(out + b) = make_int4(base, base + c4.x, base + c4.x + c4.y, base + c4.x + c4.y + c4.z);
                 }
                 run += __shfl_sync(0xffffffffu, inc, 31);
+            }
             }
             if (lane == 0) s_cnt[e] = run;
             continue;
@@ -62,29 +70,44 @@ __device__ __forceinline__ void scan_body(const int32_t *__restrict__ block_coun
         if (lane == 0) s_cnt[e] = run;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0) {
         int off = 0, poff = 0;
-        for (int e = 0; e < E; e++) {
-            int c = s_cnt[e];
-            counts[e] = c;
-            offsets[e] = off;
-            poffsets[e] = poff;
-            s_poff[e] = poff;
-            off += c;
-            poff += (c + kRowAlign - 1) / kRowAlign * kRowAlign;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            const int c = e < E ? s_cnt[e] : 0, p = (c + kRowAlign - 1) / kRowAlign * kRowAlign;
+            int ci = c, pi = p;  // inclusive sums over the lanes
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int cv = __shfl_up_sync(0xffffffffu, ci, o), pv = __shfl_up_sync(0xffffffffu, pi, o);
+                if (lane >= o) { ci += cv; pi += pv; }
+            }
+            if (e < E) {
+                counts[e] = c;
+                offsets[e] = off + ci - c;
+                poffsets[e] = s_poff[e] = poff + pi - p;
+            }
+            off += __shfl_sync(0xffffffffu, ci, 31);
+            poff += __shfl_sync(0xffffffffu, pi, 31);
         }
-        offsets[E] = off;
-        poffsets[E] = poff;
-        s_poff[E] = poff;
+        if (lane == 0) {
+            offsets[E] = off;
+            poffsets[E] = poff;
+            s_poff[E] = poff;
+        }
     }
     __syncthreads();
     const int n_tiles = s_poff[E] / kRowAlign;
     for (int i = threadIdx.x; i < max_tiles; i += blockDim.x) {
         int ex = -1;
         if (i < n_tiles) {
-            int row = i * kRowAlign;
+            const int row = i * kRowAlign;  // the last expert whose segment starts at or before it
+            int hi = E - 1;
             ex = 0;
-            while (ex + 1 < E && s_poff[ex + 1] <= row) ex++;
+            while (ex < hi) {
+                const int mid = (ex + hi + 1) >> 1;
+                if (s_poff[mid] <= row) ex = mid;
+                else hi = mid - 1;
+            }
         }
         tile_expert[i] = ex;
     }
