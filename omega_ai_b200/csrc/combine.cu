@@ -188,6 +188,7 @@ cudaError_t launch_k(omoe_handle *h, void *y, const void *resid_v, int T, cudaSt
     switch (k) {
         case 1: OMOE_COMBINE(1); break;
         case 2: OMOE_COMBINE(2); break;
+        case 3: OMOE_COMBINE(3); break;
         case 4: OMOE_COMBINE(4); break;
         case 6: OMOE_COMBINE(6); break;
         case 8: OMOE_COMBINE(8); break;
