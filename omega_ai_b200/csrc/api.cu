@@ -309,6 +309,22 @@ int omoe_create(const omoe_config *cfg, omoe_handle **out) {
     return OMOE_OK;
 }
 
+// After a host-buffer forward that was cut into chunks the routing arrays describe its last chunk.  Before they are read (or
+// the router's weights replaced) the whole batch, still staged on the device, is routed once more: logits do not depend on how
+// a batch is cut, so every array holds what one forward would have left.  No part of a forward: only read-outs pay for it.
+static int whole_batch_routing(omoe_handle *h, cudaStream_t s) {
+    if (h->whole_T == 0) return OMOE_OK;
+    const int T = h->whole_T;
+    h->last_stream = s;
+    int n = 0;
+    h->whole_T = 0;
+    CU_TRY(h, launch_router(h, h->whole_x, h->whole_io, T, s, &n));
+    if (!permute_scans(h, T)) CU_TRY(h, launch_scan(h, T, s, &n));
+    CU_TRY(h, launch_permute(h, h->whole_x, h->whole_io, T, s, &n, nullptr));
+    h->last_T = T;
+    return OMOE_OK;
+}
+
 int omoe_set_weights(omoe_handle *h, const void *w_router, const void *router_bias, const void *w_gate,
                      const void *w_up, const void *w_down, int32_t src_dtype, void *cuda_stream) {
     if (!h) return OMOE_ERR_INVALID;
@@ -317,6 +333,7 @@ int omoe_set_weights(omoe_handle *h, const void *w_router, const void *router_bi
     if (h->cfg.has_router_bias && !router_bias)
         return fail(h, OMOE_ERR_INVALID, "omoe_set_weights: the layer was created with a router bias but none was given");
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
+    if (int rc = whole_batch_routing(h, s)) return rc;  // a later read-out has to see the weights of its forward
     const int64_t E = h->cfg.n_experts, d = h->cfg.d_model, dff = h->cfg.d_ff, El = h->e_local;
     const int64_t n_exp = El * dff * d;
     // router weights and bias are always held in fp32
@@ -366,6 +383,7 @@ static int forward_impl(omoe_handle *h, const void *x_dev, int x_dtype, void *y_
                         int32_t T, cudaStream_t s, int pre) {
     NvtxRange range("omoe_forward");
     h->last_T = T;
+    h->whole_T = 0;
     h->last_io_dtype = y_dtype;
     h->last_stream = s;
     h->last_launches = 0;
@@ -523,6 +541,7 @@ int omoe_set_aux_loss(omoe_handle *h, float coef) {
 
 int omoe_get_aux_loss(omoe_handle *h, float *loss_host) {
     if (!h || !loss_host) return OMOE_ERR_INVALID;
+    if (int rc = whole_batch_routing(h, h->last_stream)) return rc;
     return bw_aux_loss(h, loss_host, h->last_stream);
 }
 
@@ -540,6 +559,8 @@ int omoe_ep_connect_local(omoe_handle **handles, int32_t world) {
 // top-2 in one piece 478 us, in two 392 us.
 static bool chunk_pays(omoe_handle *h, int T, int chunks, size_t row_bytes) {
     if (h->cfg.world != 1 || h->cfg.compute_dtype != OMOE_BF16 || h->host_chunk_min >= 1 << 30) return false;
+    // a backward follows a forward of the whole batch, and stage times are a forward's
+    if (bw_training(h) || h->profiling) return false;
     const long rows = (long)(T / chunks) * h->cfg.top_k;
     return (size_t)(T / chunks) * row_bytes >= (size_t)4 << 20 && rows >= 512l * h->cfg.n_experts &&
            !experts_split_k(h, rows);
@@ -586,6 +607,7 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
                                       cudaMemcpyHostToDevice, h->copy_in));
         CU_TRY(h, cudaEventRecord(h->ev_in[i], h->copy_in));
     }
+    int launches = 0;
     for (int i = 0; i < chunks; i++) {
         const int t0 = i * per, n = t0 >= T ? 0 : ((t0 + per <= T) ? per : T - t0);
         const size_t off = (size_t)(n > 0 ? t0 : 0) * row_bytes;
@@ -593,6 +615,7 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
         if (n > 0 || h->cfg.world > 1) {
             int rc = omoe_forward(h, xs + off, ys + off, n, io_dtype, s);
             if (rc != OMOE_OK) return rc;
+            launches += h->last_launches;
         }
         CU_TRY(h, cudaEventRecord(h->ev_out[i], s));
         CU_TRY(h, cudaStreamWaitEvent(h->copy_out, h->ev_out[i], 0));
@@ -604,6 +627,12 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
     CU_TRY(h, cudaEventRecord(h->ev_set_d2h[set], h->copy_out));
     h->last_stream = s;
     h->host_pending = true;
+    if (chunks > 1 && h->cfg.world == 1) {
+        h->last_launches = launches;
+        h->whole_x = xs;
+        h->whole_T = T;
+        h->whole_io = io_dtype;
+    }
     return OMOE_OK;
 }
 
@@ -649,6 +678,7 @@ int omoe_forward_host(omoe_handle *h, const void *x_host, void *y_host, int32_t 
 int omoe_get_routing(omoe_handle *h, int32_t *topk_idx, float *topk_w, int32_t *counts, int32_t *offsets,
                      int32_t *perm) {
     if (!h) return OMOE_ERR_INVALID;
+    if (int rc = whole_batch_routing(h, h->last_stream)) return rc;
     const int T = h->last_T, k = h->cfg.top_k, E = h->cfg.n_experts;
     cudaStream_t s = h->last_stream;
     if (perm && T > 0) CU_TRY(h, launch_perm_readout(h, T, s));
@@ -671,6 +701,7 @@ int omoe_get_routing(omoe_handle *h, int32_t *topk_idx, float *topk_w, int32_t *
 
 int omoe_get_logits(omoe_handle *h, float *logits) {
     if (!h || !logits) return OMOE_ERR_INVALID;
+    if (int rc = whole_batch_routing(h, h->last_stream)) return rc;
     CU_TRY(h, cudaStreamSynchronize(h->last_stream));
     const size_t n = (size_t)h->last_T * h->cfg.n_experts;
     if (n) CU_TRY(h, cudaMemcpy(logits, h->logits, n * 4, cudaMemcpyDeviceToHost));
