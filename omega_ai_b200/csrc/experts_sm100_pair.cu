@@ -61,15 +61,17 @@ struct PairCfg {
 };
 constexpr int kTableInts = 3 * kMaxExperts + 2;   // token-tile prefix, counts, first rows of the local experts; narrow step
 constexpr int kBarBytesP = 256;
-// A step whose experts hold at most 64 rows each is bound by the weights' way from HBM: its stages need room for 32 token rows per
-// CTA, not 128, and nine of those take the ring's place (64 tokens, d 4096, d_ff 14336, 8 experts: 494 -> 479 us; 8 tokens, d 2048,
-// 64 experts: 124.3 -> 122.1 us.  Requesting the two halves of a weight row's 256 bytes together instead: 3 % slower.)
+// A step whose experts hold at most 64 (128) rows each is bound by the weights' way from HBM: its stages need room for 32 (64)
+// token rows per CTA, not 128, and nine (eight) of those take the ring's place (64 tokens, d 4096, d_ff 14336, 8 experts: 494 ->
+// 479 us; 8 tokens, d 2048, 64 experts: 124.3 -> 122.1 us; 256 tokens of the first layer: 517 -> 502 us.  Requesting the two
+// halves of a weight row's 256 bytes together instead: 3 % slower.)
 constexpr int kStagesNarrow = 9, kStageBytesNarrow = kABytesP + 4096;
+constexpr int kStagesMid = 8, kStageBytesMid = kABytesP + 8192;
 template <PairKind KIND>
 constexpr int pair_smem_bytes() {
     return PairCfg<KIND>::kStages * kStageBytesP + PairCfg<KIND>::kParts * PairCfg<KIND>::kPartBytes + kBarBytesP + kTableInts * 4 + 1024 /*align slack*/;
 }
-static_assert(kStagesNarrow * kStageBytesNarrow <= 6 * kStageBytesP, "the narrow ring lies in the wide one's place");
+static_assert(kStagesNarrow * kStageBytesNarrow <= 6 * kStageBytesP && kStagesMid * kStageBytesMid <= 6 * kStageBytesP, "the narrow rings lie in the wide one's place");
 static_assert(pair_smem_bytes<PairKind::kUpGate>() <= 227 * 1024 && pair_smem_bytes<PairKind::kUpGateKeep>() <= 227 * 1024 &&
                   pair_smem_bytes<PairKind::kSwigluBack>() <= 227 * 1024,
               "shared memory of one CTA");
@@ -160,7 +162,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
         most = __reduce_max_sync(0xffffffffu, most);
         if (lane == 0) {
             s_tt[E] = run;
-            *s_narrow = most <= 64;
+            *s_narrow = most <= 64 ? 2 : (most <= 128 ? 1 : 0);
         }
     }
     tc_fence_before();
@@ -168,8 +170,9 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const bool narrow = kRingStages == 6 && *s_narrow != 0;
-    const int kStagesP = narrow ? kStagesNarrow : kRingStages, stage_bytes = narrow ? kStageBytesNarrow : kStageBytesP;
+    const int narrow = kRingStages == 6 ? *s_narrow : 0;
+    const int kStagesP = narrow == 2 ? kStagesNarrow : (narrow == 1 ? kStagesMid : kRingStages);
+    const int stage_bytes = narrow == 2 ? kStageBytesNarrow : (narrow == 1 ? kStageBytesMid : kStageBytesP);
     const int token_tiles = s_tt[E];
     const int n_ft = (n_out + kFeatPair - 1) / kFeatPair;
     const int total = token_tiles * n_ft;
