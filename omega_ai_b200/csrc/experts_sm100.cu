@@ -14,6 +14,8 @@
 // accumulator with tcgen05.ld while the next tile's mainloop already runs in
 // the other half of tensor memory.
 //
+// On one GPU most steps run on experts_sm100_pair.cu instead; launch_experts_bf16 has the rule.
+//
 // Every wait on an mbarrier is bounded: when it runs out the kernel raises a
 // flag in the device error word, lets outstanding copies land, frees its tensor
 // memory and returns, so the context stays usable.

@@ -15,7 +15,8 @@
 //
 // Measured against the kernel of experts_sm100.cu (128 x 256 tiles, one CTA each), whole layer: 16384 tokens, d 4096,
 // d_ff 14336, 8 experts top-2 10.27 -> 9.92 ms; 1531 tokens, d 1544, d_ff 4104, 12 experts top-3 355 -> 306 us; 4096
-// tokens on d 1024, d_ff 2816 the same within 1 %.  That kernel stays for expert parallelism, whose rows it waits for and sends.
+// tokens on d 1024, d_ff 2816 the same within 1 %.  That kernel stays for expert
+// parallelism, whose rows it waits for and sends, and for a down product that it runs in one round (launch_experts_bf16).
 //
 // The accumulator comes out transposed (tensor-memory lane = output feature, column = token).  For up/gate the A tile
 // interleaves 8 gate rows with 8 up rows (one 4-D tensor map over both matrices, which lie back to back), so
