@@ -135,6 +135,12 @@ wgrad_kernel(const __grid_constant__ WgradMaps maps, int n_mat, int M, int N, co
                     if (++stage == kStagesW) { stage = 0; phase ^= 1u; }
                 }
             }
+            // The issuer's commits arrive in both CTAs, in their own time: every stage's last one has to be in before this CTA may
+            // go (the cluster barrier at the end orders the threads' arrivals, not those of the tensor core).
+            for (int i = 0; ok && i < kStagesW; i++) {
+                ok = warp_wait(empty_bar(stage), phase ^ 1u, abort_flag, dev_err);
+                if (++stage == kStagesW) { stage = 0; phase ^= 1u; }
+            }
             if (!ok) {
                 // let copies that were already issued land before the CTA retires
                 const unsigned long long t0 = globaltimer_ns();
