@@ -434,7 +434,7 @@ static int forward_impl(omoe_handle *h, const void *x_dev, int x_dtype, void *y_
     } else if (h->cfg.compute_dtype == OMOE_BF16) {
         CU_TRY(h, launch_experts_bf16(h, s, &n, prof ? h->ev[5] : nullptr, (long)T * h->cfg.top_k));
     } else {
-        CU_TRY(h, launch_experts_f32(h, s, &n));
+        CU_TRY(h, launch_experts_f32(h, s, &n, (long)T * h->cfg.top_k));
         MARK(5);
     }
     MARK(6);

@@ -347,9 +347,12 @@ zero_pad_rows_kernel(__nv_bfloat16 *__restrict__ buf, int ld, const int32_t *__r
 // first access.  One GPU only: with expert parallelism kernels without the instructions stand in between.
 bool bw_pdl(const omoe_handle *h) { return h->pdl && h->cfg.world == 1; }
 
-cudaError_t forward_experts(omoe_handle *h, BwState *b, cudaStream_t s, int *n) {
+// Rows of the step, where this rank alone decides them.
+long step_rows(const omoe_handle *h, int T) { return h->cfg.world == 1 ? (long)T * h->cfg.top_k : -1; }
+
+cudaError_t forward_experts(omoe_handle *h, BwState *b, int T, cudaStream_t s, int *n) {
     const int d = h->cfg.d_model, dff = h->cfg.d_ff;
-    if (h->cfg.compute_dtype != OMOE_BF16) return f32_forward_experts(h, s, b->gu, n);
+    if (h->cfg.compute_dtype != OMOE_BF16) return f32_forward_experts(h, s, step_rows(h, T), b->gu, n);
     // padding rows hold rows of earlier steps: zero them, so that g, u and h are zero there too and a
     // reduction over blocks of 64 rows (the weight gradients) adds nothing
     const bool pdl = bw_pdl(h);
@@ -405,7 +408,7 @@ cudaError_t backward_t(omoe_handle *h, BwState *b, const void *x, bool x_is_comp
         *n += 2;
     } else {
         // dg | du from dyp * W_down, then dxp = dg * W_gate + du * W_up
-        BW_TRY(f32_grad_rows(h, s, b->dyp, b->gu, b->dgu, b->dxp, n));
+        BW_TRY(f32_grad_rows(h, s, step_rows(h, T), b->dyp, b->gu, b->dgu, b->dxp, n));
         if (ep) {
             BW_TRY(ep_signal_out(h, s));
             (*n)++;
@@ -561,7 +564,7 @@ void bw_forward_empty(omoe_handle *h) {
 
 cudaError_t bw_forward_experts(omoe_handle *h, int T, cudaStream_t s, int *n) {
     BwState *b = static_cast<BwState *>(h->bw);
-    cudaError_t e = forward_experts(h, b, s, n);
+    cudaError_t e = forward_experts(h, b, T, s, n);
     b->fwd_valid = e == cudaSuccess;
     b->fwd_T = T;
     return e;

@@ -33,10 +33,10 @@ struct alignas(64) WgradMaps {
 };
 cudaError_t launch_wgrad(omoe_handle *h, cudaStream_t s, const WgradMaps &maps, int n_mat, int M, int N);
 
-// fp32 layers (experts_f32.cu).  Forward products: h = silu(g) * u and yp, keeping g | u in gu unless null.
-cudaError_t f32_forward_experts(omoe_handle *h, cudaStream_t s, void *gu, int *n);
+// fp32 layers (experts_f32.cu); rows as for launch_experts_f32.  Forward products: h = silu(g) * u and yp, keeping g | u in gu unless null.
+cudaError_t f32_forward_experts(omoe_handle *h, cudaStream_t s, long rows, void *gu, int *n);
 // dgu = dg | du and dxp from the gradient dyp of the expert outputs.
-cudaError_t f32_grad_rows(omoe_handle *h, cudaStream_t s, const void *dyp, void *gu, void *dgu, void *dxp, int *n);
+cudaError_t f32_grad_rows(omoe_handle *h, cudaStream_t s, long rows, const void *dyp, void *gu, void *dgu, void *dxp, int *n);
 // out_z [e_local, M, N] = (a + z*a_next)^T * b over each expert's rows, z < n_mat; a has lda floats between rows.
 cudaError_t f32_wgrad(omoe_handle *h, cudaStream_t s, const void *a, int lda, int a_next, const void *b, int n_mat, int M,
                       int N, float *out0, float *out1);

@@ -181,7 +181,8 @@ cudaError_t launch_combine(omoe_handle *h, void *y, int io_dtype, int T, cudaStr
 // xn = (x / rms(x)) * gamma per row, in the layer's compute dtype (the block's pre-FFN RMSNorm).
 cudaError_t launch_rmsnorm(omoe_handle *h, const void *x, int x_dtype, const float *gamma, float eps, int T,
                            cudaStream_t s, int *n);
-cudaError_t launch_experts_f32(omoe_handle *h, cudaStream_t s, int *n);
+// rows: how many rows the step has on this rank, negative where that is not known
+cudaError_t launch_experts_f32(omoe_handle *h, cudaStream_t s, int *n, long rows);
 // rows_ub: upper bound on the rows (token, expert picks) this GPU's experts hold in the step, -1 if unknown; a small
 // bound sends a product with few tiles to the split-K kernels
 // gate: expert parallel only -- the up/gate product waits for the dispatched rows, the down product raises

@@ -691,7 +691,7 @@ int ep_forward(omoe_handle *h, const void *x, int x_dtype, void *y, int y_dtype,
         TRY(launch_experts_bf16(h, s, &n, prof ? h->ev[5] : nullptr, (long)h->cfg.t_max * W * h->cfg.top_k,
                                 gated ? &gate : nullptr));
     } else {
-        TRY(launch_experts_f32(h, s, &n));
+        TRY(launch_experts_f32(h, s, &n, -1));
         MARK(5);
     }
     MARK(6);

@@ -13,8 +13,12 @@
 // padding rows (32 rows x 64 columns, 128 threads, 4 x 4 outputs each), operands brought by 16-byte asynchronous
 // copies into a ring of three stages so that the loads of two steps are always under way, and both halves of a
 // gate/up pair in one block.  Measured against 64 x 64 tiles that loaded, waited and multiplied in turn and walked the padding
-// rows in the backward: forward of 64 tokens, d 128, d_ff 256, 8 experts 45.5 -> 35.7 us; training step of 300 tokens,
-// d 256, d_ff 384 452 -> 256 us.  Every output is one chain of fused multiply-adds over ascending k.
+// rows in the backward: forward of 64 tokens, d 128, d_ff 256, 8 experts 44.4 -> 27.5 us; training step of 300 tokens,
+// d 256, d_ff 384 497 -> 181 us.  Every output is one chain of fused multiply-adds over ascending k.
+//
+// Blocks are numbered over the row tiles that hold rows, as many as the step's rows can give: a grid over the buffers' rows made
+// blocks without rows hold their slots until the product before was done, and had the real ones share the SMs that were left
+// (256 tokens, d 512, d_ff 1024, 8 experts top-2: 158 us, now 109; 48 tiles of which 20 hold rows).
 #include "backward.cuh"
 #include "common.cuh"
 
@@ -50,28 +54,45 @@ enum Epi {
     kSum,         // c = A B0 + A1 B1
 };
 
-// Rows grouped by expert: the expert of a row comes from its 128-row tile.  B is [expert][n][k] (B_KN false) or
+// Rows grouped by expert, row tiles numbered over the experts in order, column tiles fastest.  B is [expert][n][k] (B_KN false) or
 // [expert][k][n]; A1 starts a_next floats after A.
 template <bool B_KN, Epi EPI>
 __global__ void __launch_bounds__(128)
 rows_sgemm_kernel(const float *__restrict__ A, int lda, int a_next, const float *__restrict__ B0,
                   const float *__restrict__ B1, float *__restrict__ C, float *__restrict__ gu, int N, int K,
-                  const int32_t *__restrict__ tile_expert, const int32_t *__restrict__ poffsets,
-                  const int32_t *__restrict__ counts, int E) {
+                  const int32_t *__restrict__ poffsets, const int32_t *__restrict__ counts, int E) {
     constexpr int NS = (EPI == kStore || EPI == kSwigluBack) ? 1 : 2;  // accumulator sets
     constexpr int NA = EPI == kSum ? 2 : 1;
     constexpr int B_WORDS = B_KN ? BK * LDN : BN * LDK;
     __shared__ __align__(16) float sa[ST][NA][BM * LDK];
     __shared__ __align__(16) float sb[ST][NS][B_WORDS];
-    pdl_trigger();
     pdl_wait();
-    const int row0 = blockIdx.y * BM;
-    if (row0 >= poffsets[E]) return;
-    const int e = tile_expert[row0 / kRowAlign];
-    const int valid = poffsets[e] + counts[e] - row0;  // rows of this tile that carry tokens
-    if (valid <= 0) return;
-    const int n0 = blockIdx.x * BN;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int n_ct = (N + BN - 1) / BN, rt = blockIdx.x / n_ct, n0 = (blockIdx.x - rt * n_ct) * BN;
+    // the expert of row tile rt, ceil(count / BM) tiles each; every warp works it out for itself
+    int e = -1, tile = 0, cnt = 0, before = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+        const int lane = tid & 31;
+        const int c = e0 + lane < E ? counts[e0 + lane] : 0, own = (c + BM - 1) / BM;
+        int upto = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        upto += before;
+        const uint32_t hit = __ballot_sync(0xffffffffu, rt >= upto - own && rt < upto);
+        if (hit != 0) {
+            const int src = __ffs(hit) - 1;
+            e = e0 + src;
+            tile = rt - __shfl_sync(0xffffffffu, upto - own, src);
+            cnt = __shfl_sync(0xffffffffu, c, src);
+            break;
+        }
+        before = __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (e < 0) return;
+    const int row0 = poffsets[e] + tile * BM, valid = cnt - tile * BM;  // rows of this tile that carry tokens: > 0
     const float *Bs[2] = {B0 + (size_t)e * N * K, NS == 2 ? B1 + (size_t)e * N * K : nullptr};
 
     auto issue = [&](int step) {
@@ -149,6 +170,7 @@ rows_sgemm_kernel(const float *__restrict__ A, int lda, int a_next, const float 
             }
         }
     }
+    pdl_trigger();  // not before: a block of the next product that waits here takes this one's place
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int r = ty * 4 + i;
@@ -233,36 +255,54 @@ wgrad_sgemm_kernel(const float *__restrict__ A, int lda, int a_next, const float
     }
 }
 
+// Most row tiles any placement of a step's rows on the local experts can give; `rows` is negative where only the capacity of
+// the buffers bounds them.
+long row_tiles(const omoe_handle *h, long rows) {
+    if (rows < 0) return h->rows_cap / BM;
+    const long some = rows < h->e_local ? rows : h->e_local;  // experts that can have a row
+    return some + (rows - some) / BM;
+}
+
+// Dependent launch hides about 3.5 us per forward, but the blocks of the next product then settle, several to an SM, wherever
+// the product before them finishes first, and stay there while the other SMs go idle.  That costs nothing while all blocks are
+// fewer than the SMs by a margin: it is used up to two thirds of the SMs.  Forward with it and without: 44 blocks (256 tokens, d 128,
+// d_ff 256, 4 experts top-1) 27.9 us against 31.0; 92 (8 experts top-2) 31.8 against 31.7; 140 (1024 tokens, 4 experts) 40.6 against 33.0;
+// 368 (256 tokens, d 512, d_ff 1024, 8 experts top-2) 121 against 110.
+bool dependent_launch(const omoe_handle *h, long rows) {
+    const int widest = h->cfg.d_model > h->cfg.d_ff ? h->cfg.d_model : h->cfg.d_ff;
+    return h->pdl && h->cfg.world == 1 && row_tiles(h, rows) * ceil_div(widest, BN) * 3 <= 2 * (long)h->sm_count;
+}
+
 template <bool B_KN, Epi EPI>
-cudaError_t launch_rows(omoe_handle *h, cudaStream_t s, const void *A, int lda, int a_next, const void *B0, const void *B1,
-                        void *C, void *gu, int N, int K) {
-    return launch_ex(rows_sgemm_kernel<B_KN, EPI>, dim3(ceil_div(N, BN), (unsigned)(h->rows_cap / BM)), dim3(128), 0, s,
-                     h->pdl && h->cfg.world == 1, static_cast<const float *>(A), lda, a_next, static_cast<const float *>(B0),
+cudaError_t launch_rows(omoe_handle *h, cudaStream_t s, long rows, const void *A, int lda, int a_next, const void *B0,
+                        const void *B1, void *C, void *gu, int N, int K) {
+    return launch_ex(rows_sgemm_kernel<B_KN, EPI>, dim3((unsigned)(row_tiles(h, rows) * ceil_div(N, BN))), dim3(128), 0, s,
+                     dependent_launch(h, rows), static_cast<const float *>(A), lda, a_next, static_cast<const float *>(B0),
                      static_cast<const float *>(B1), static_cast<float *>(C), static_cast<float *>(gu), N, K,
-                     h->ex_tile_expert, h->ex_poffsets, h->ex_counts, h->e_local);
+                     h->ex_poffsets, h->ex_counts, h->e_local);
 }
 
 }  // namespace
 
-cudaError_t f32_forward_experts(omoe_handle *h, cudaStream_t s, void *gu, int *n) {
+cudaError_t f32_forward_experts(omoe_handle *h, cudaStream_t s, long rows, void *gu, int *n) {
     const int d = h->cfg.d_model, dff = h->cfg.d_ff;
-    cudaError_t e = gu ? launch_rows<false, kSwigluKeep>(h, s, h->xp, d, 0, h->w_gate, h->w_up, h->hbuf, gu, dff, d)
-                       : launch_rows<false, kSwiglu>(h, s, h->xp, d, 0, h->w_gate, h->w_up, h->hbuf, nullptr, dff, d);
+    cudaError_t e = gu ? launch_rows<false, kSwigluKeep>(h, s, rows, h->xp, d, 0, h->w_gate, h->w_up, h->hbuf, gu, dff, d)
+                       : launch_rows<false, kSwiglu>(h, s, rows, h->xp, d, 0, h->w_gate, h->w_up, h->hbuf, nullptr, dff, d);
     if (e != cudaSuccess) return e;
     (*n)++;
-    e = launch_rows<false, kStore>(h, s, h->hbuf, dff, 0, h->w_down, nullptr, h->yp, nullptr, d, dff);
+    e = launch_rows<false, kStore>(h, s, rows, h->hbuf, dff, 0, h->w_down, nullptr, h->yp, nullptr, d, dff);
     if (e == cudaSuccess) (*n)++;
     return e;
 }
 
-cudaError_t launch_experts_f32(omoe_handle *h, cudaStream_t s, int *n) { return f32_forward_experts(h, s, nullptr, n); }
+cudaError_t launch_experts_f32(omoe_handle *h, cudaStream_t s, int *n, long rows) { return f32_forward_experts(h, s, rows, nullptr, n); }
 
-cudaError_t f32_grad_rows(omoe_handle *h, cudaStream_t s, const void *dyp, void *gu, void *dgu, void *dxp, int *n) {
+cudaError_t f32_grad_rows(omoe_handle *h, cudaStream_t s, long rows, const void *dyp, void *gu, void *dgu, void *dxp, int *n) {
     const int d = h->cfg.d_model, dff = h->cfg.d_ff;
-    cudaError_t e = launch_rows<true, kSwigluBack>(h, s, dyp, d, 0, h->w_down, nullptr, dgu, gu, dff, d);
+    cudaError_t e = launch_rows<true, kSwigluBack>(h, s, rows, dyp, d, 0, h->w_down, nullptr, dgu, gu, dff, d);
     if (e != cudaSuccess) return e;
     (*n)++;
-    e = launch_rows<true, kSum>(h, s, dgu, 2 * dff, dff, h->w_gate, h->w_up, dxp, nullptr, d, dff);
+    e = launch_rows<true, kSum>(h, s, rows, dgu, 2 * dff, dff, h->w_gate, h->w_up, dxp, nullptr, d, dff);
     if (e == cudaSuccess) (*n)++;
     return e;
 }
