@@ -404,7 +404,7 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                             out(stg + 2 * kPass * 128, u);
                         }
 #pragma unroll
-                        for (int i = 0; i < 16; i++) g[i] = silu_f(g[i]) * u[i];
+                        for (int i = 0; i < 16; i++) g[i] = (kOuts == 3 ? silu_full(g[i]) : silu_f(g[i])) * u[i];
                         out(stg, g);
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -452,8 +452,8 @@ pair_gemm_kernel(const __grid_constant__ PairMaps maps, int n_out, int K, const 
                             for (int q = 0; q < 2; q++) {
                                 auto half_of = [&](uint32_t w) { return __uint_as_float(q ? w & 0xffff0000u : w << 16); };
                                 const float x = half_of(g), d = half_of(dh);
-                                const float sg = __fdividef(1.0f, 1.0f + __expf(-x));
-                                du[q] = d * (x * sg);
+                                const float den = 1.0f + expf(-x), sg = 1.0f / den;
+                                du[q] = d * (x / den);
                                 dg[q] = (d * half_of(u)) * (sg * (1.0f + x * (1.0f - sg)));
                             }
                             asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(pack_bf16(dg[0], dg[1])) : "memory");

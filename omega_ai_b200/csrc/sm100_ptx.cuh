@@ -149,7 +149,11 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BLO
                             ((uint32_t)(BLOCK_M >> 4) << 24);
 
 // x / (1 + exp(-x)) with the fast exponential and reciprocal (the result is rounded to bf16 next)
+// The inference epilogues' SiLU: the exponential's error grows with |x| (2 + 1.16 |x| units in the last place) and the quotient is
+// zero below x = -87.3, where exp(-x) passes 2^126.
 __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
+// A training step's SiLU, in the forward and where it is differentiated: exponential and division of full fp32 accuracy.
+__device__ __forceinline__ float silu_full(float x) { return x / (1.0f + expf(-x)); }
 
 
 }  // namespace sm100
