@@ -137,7 +137,10 @@ OMOE_API int omoe_forward_block(omoe_handle *h, const void *x_dev, const float *
  * forward, D2H copy of y, then a stream synchronise so y is readable on return.
  * On one GPU a batch of 8192 tokens or more is cut into chunks of at least 4096 whose
  * copies overlap the kernels of their neighbours (tokens are independent, so
- * y is bit-identical); the routing read-outs then describe the last chunk.
+ * y is bit-identical); the routing read-outs and the launch count then describe
+ * the last chunk.  A smaller batch or a chunk may run as several forwards where
+ * that is faster (not in training mode): what is read out afterwards is that of
+ * the whole of it.
  * With world > 1 the call is collective like omoe_forward, and the batch is cut
  * too: into as many chunks (at most 8, of at least 512 tokens) as t_max allows,
  * the same number on every rank, each chunk one collective forward.

@@ -309,22 +309,6 @@ int omoe_create(const omoe_config *cfg, omoe_handle **out) {
     return OMOE_OK;
 }
 
-// After a host-buffer forward that was cut into chunks the routing arrays describe its last chunk.  Before they are read (or
-// the router's weights replaced) the whole batch, still staged on the device, is routed once more: logits do not depend on how
-// a batch is cut, so every array holds what one forward would have left.  No part of a forward: only read-outs pay for it.
-static int whole_batch_routing(omoe_handle *h, cudaStream_t s) {
-    if (h->whole_T == 0) return OMOE_OK;
-    const int T = h->whole_T;
-    h->last_stream = s;
-    int n = 0;
-    h->whole_T = 0;
-    CU_TRY(h, launch_router(h, h->whole_x, h->whole_io, T, s, &n));
-    if (!permute_scans(h, T)) CU_TRY(h, launch_scan(h, T, s, &n));
-    CU_TRY(h, launch_permute(h, h->whole_x, h->whole_io, T, s, &n, nullptr));
-    h->last_T = T;
-    return OMOE_OK;
-}
-
 int omoe_set_weights(omoe_handle *h, const void *w_router, const void *router_bias, const void *w_gate,
                      const void *w_up, const void *w_down, int32_t src_dtype, void *cuda_stream) {
     if (!h) return OMOE_ERR_INVALID;
@@ -333,7 +317,6 @@ int omoe_set_weights(omoe_handle *h, const void *w_router, const void *router_bi
     if (h->cfg.has_router_bias && !router_bias)
         return fail(h, OMOE_ERR_INVALID, "omoe_set_weights: the layer was created with a router bias but none was given");
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-    if (int rc = whole_batch_routing(h, s)) return rc;  // a later read-out has to see the weights of its forward
     const int64_t E = h->cfg.n_experts, d = h->cfg.d_model, dff = h->cfg.d_ff, El = h->e_local;
     const int64_t n_exp = El * dff * d;
     // router weights and bias are always held in fp32
@@ -383,7 +366,7 @@ static int forward_impl(omoe_handle *h, const void *x_dev, int x_dtype, void *y_
                         int32_t T, cudaStream_t s, int pre) {
     NvtxRange range("omoe_forward");
     h->last_T = T;
-    h->whole_T = 0;
+    h->picks_only = false;
     h->last_io_dtype = y_dtype;
     h->last_stream = s;
     h->last_launches = 0;
@@ -534,6 +517,20 @@ int omoe_get_weight_grads(omoe_handle *h, float *d_router, float *d_router_bias,
     return check_dev_err(h);
 }
 
+// The picks of the last_T rows that the read-outs describe, in a malloc'ed array (the caller frees it), and how many fell on
+// every expert.
+static int read_picks(omoe_handle *h, int32_t **idx, int32_t *counts) {
+    const size_t n = (size_t)h->last_T * h->cfg.top_k;
+    CU_TRY(h, cudaStreamSynchronize(h->last_stream));
+    int32_t *v = static_cast<int32_t *>(malloc(n * 4 + 4));
+    *idx = v;
+    if (!v) return fail(h, OMOE_ERR_NOMEM, "host allocation failed");
+    CU_TRY(h, cudaMemcpy(v, h->topk_idx, n * 4, cudaMemcpyDeviceToHost));
+    memset(counts, 0, sizeof(int32_t) * h->cfg.n_experts);
+    for (size_t f = 0; f < n; f++) counts[v[f]]++;
+    return OMOE_OK;
+}
+
 int omoe_set_aux_loss(omoe_handle *h, float coef) {
     if (!h) return OMOE_ERR_INVALID;
     return bw_set_aux(h, coef);
@@ -541,8 +538,14 @@ int omoe_set_aux_loss(omoe_handle *h, float coef) {
 
 int omoe_get_aux_loss(omoe_handle *h, float *loss_host) {
     if (!h || !loss_host) return OMOE_ERR_INVALID;
-    if (int rc = whole_batch_routing(h, h->last_stream)) return rc;
-    return bw_aux_loss(h, loss_host, h->last_stream);
+    int32_t counts[kMaxExperts];
+    if (h->picks_only) {
+        int32_t *idx = nullptr;
+        const int rc = read_picks(h, &idx, counts);
+        free(idx);
+        if (rc != OMOE_OK) return rc;
+    }
+    return bw_aux_loss(h, loss_host, h->last_stream, h->picks_only ? counts : nullptr);
 }
 
 int omoe_ep_connect_local(omoe_handle **handles, int32_t world) {
@@ -552,15 +555,29 @@ int omoe_ep_connect_local(omoe_handle **handles, int32_t world) {
     return ep_connect_local(handles, world);
 }
 
+// Chunk i of a host batch of T rows cut into pieces * sub: its first row, its rows and its piece's first row.
+struct HostChunk {
+    int t0, n, piece0;
+};
+static HostChunk host_chunk(int T, int pieces, int sub, int i) {
+    auto part = [](int n, int parts, int j) {  // part j of n rows: first row, rows
+        const int per = (n + parts - 1) / parts, first = j * per < n ? j * per : n;
+        return HostChunk{first, first + per <= n ? per : n - first, 0};
+    };
+    const HostChunk p = part(T, pieces, i / sub), c = part(p.n, sub, i % sub);
+    return HostChunk{p.t0 + c.t0, c.n, p.t0};
+}
+
 // One GPU, batches below host_chunk_min per chunk: whether cutting into `chunks` still pays.  A chunk's copy has to
 // outlast the fixed part of one more forward (4 MB is about 75 us over PCIe against 45 us), its products have to stay bound by arithmetic and not by
 // reading the weights once more (512 rows per expert are twice the rows at which the two take the same time), and they have
 // to run on the same kernels as the whole batch's, so that every row keeps its bits.  Measured: 4096 tokens, d 1024, d_ff 2816, 8 experts
 // top-2 in one piece 478 us, in two 392 us.
-static bool chunk_pays(omoe_handle *h, int T, int chunks, size_t row_bytes) {
+static bool chunk_pays(omoe_handle *h, int T, int pieces, int sub, size_t row_bytes) {
     if (h->cfg.world != 1 || h->cfg.compute_dtype != OMOE_BF16 || h->host_chunk_min >= 1 << 30) return false;
     // a backward follows a forward of the whole batch, and stage times are a forward's
     if (bw_training(h) || h->profiling) return false;
+    const int chunks = pieces * sub;
     const long rows = (long)(T / chunks) * h->cfg.top_k;
     return (size_t)(T / chunks) * row_bytes >= (size_t)4 << 20 && rows >= 512l * h->cfg.n_experts &&
            !experts_split_k(h, rows);
@@ -583,13 +600,16 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
                                 cudaStream_t s, bool chunked) {
     NvtxRange range("omoe_forward_host");
     const size_t row_bytes = (size_t)h->cfg.d_model * elt_size(io_dtype);
-    int chunks = 1;
+    // `pieces` is the cut the interface states: the read-outs describe the last one.  Each may be cut further into `sub` forwards,
+    // which nothing but the launch count shows.
+    int pieces = 1, sub = 1;
     if (chunked) {
         const int basis = h->cfg.world == 1 ? T : h->cfg.t_max;
         const int cmin = h->cfg.world == 1 ? h->host_chunk_min : h->host_chunk_min_ep;
-        while (chunks < kHostChunksMax && (basis / (chunks * 2) >= cmin || chunk_pays(h, T, chunks * 2, row_bytes))) chunks *= 2;
+        while (pieces < kHostChunksMax && basis / (pieces * 2) >= cmin) pieces *= 2;
+        while (pieces * sub < kHostChunksMax && chunk_pays(h, T, pieces, sub * 2, row_bytes)) sub *= 2;
     }
-    const int per = (T + chunks - 1) / chunks;
+    const int chunks = pieces * sub;
     const int set = h->stage_next;
     h->stage_next ^= 1;
     char *xs = static_cast<char *>(h->x_stage[set]), *ys = static_cast<char *>(h->y_stage[set]);
@@ -600,22 +620,34 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
     CU_TRY(h, cudaStreamWaitEvent(h->copy_in, h->ev_set_fwd[set], 0));
     CU_TRY(h, cudaStreamWaitEvent(s, h->ev_set_d2h[set], 0));
     for (int i = 0; i < chunks; i++) {
-        const int t0 = i * per, n = t0 >= T ? 0 : ((t0 + per <= T) ? per : T - t0);
+        const auto [t0, n, piece0] = host_chunk(T, pieces, sub, i);
         const size_t off = (size_t)t0 * row_bytes;
         if (n > 0)
             CU_TRY(h, cudaMemcpyAsync(xs + off, static_cast<const char *>(x_host) + off, (size_t)n * row_bytes,
                                       cudaMemcpyHostToDevice, h->copy_in));
         CU_TRY(h, cudaEventRecord(h->ev_in[i], h->copy_in));
     }
-    int launches = 0;
+    int launches = 0, described = 0;
     for (int i = 0; i < chunks; i++) {
-        const int t0 = i * per, n = t0 >= T ? 0 : ((t0 + per <= T) ? per : T - t0);
+        const auto [t0, n, piece0] = host_chunk(T, pieces, sub, i);
         const size_t off = (size_t)(n > 0 ? t0 : 0) * row_bytes;
         CU_TRY(h, cudaStreamWaitEvent(s, h->ev_in[i], 0));
         if (n > 0 || h->cfg.world > 1) {
-            int rc = omoe_forward(h, xs + off, ys + off, n, io_dtype, s);
+            // the chunks of a piece leave their logits, picks and gate weights side by side
+            const size_t row = n > 0 ? t0 - piece0 : 0;
+            float *const logits = h->logits, *const topk_w = h->topk_w;
+            int32_t *const topk_idx = h->topk_idx;
+            h->logits += row * h->cfg.n_experts;
+            h->topk_w += row * h->cfg.top_k;
+            h->topk_idx += row * h->cfg.top_k;
+            const int rc = omoe_forward(h, xs + off, ys + off, n, io_dtype, s);
+            h->logits = logits;
+            h->topk_w = topk_w;
+            h->topk_idx = topk_idx;
             if (rc != OMOE_OK) return rc;
+            if (row == 0) launches = described = 0;
             launches += h->last_launches;
+            described += n;
         }
         CU_TRY(h, cudaEventRecord(h->ev_out[i], s));
         CU_TRY(h, cudaStreamWaitEvent(h->copy_out, h->ev_out[i], 0));
@@ -627,11 +659,10 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
     CU_TRY(h, cudaEventRecord(h->ev_set_d2h[set], h->copy_out));
     h->last_stream = s;
     h->host_pending = true;
-    if (chunks > 1 && h->cfg.world == 1) {
+    if (sub > 1) {
         h->last_launches = launches;
-        h->whole_x = xs;
-        h->whole_T = T;
-        h->whole_io = io_dtype;
+        h->last_T = described;
+        h->picks_only = true;
     }
     return OMOE_OK;
 }
@@ -678,10 +709,9 @@ int omoe_forward_host(omoe_handle *h, const void *x_host, void *y_host, int32_t 
 int omoe_get_routing(omoe_handle *h, int32_t *topk_idx, float *topk_w, int32_t *counts, int32_t *offsets,
                      int32_t *perm) {
     if (!h) return OMOE_ERR_INVALID;
-    if (int rc = whole_batch_routing(h, h->last_stream)) return rc;
     const int T = h->last_T, k = h->cfg.top_k, E = h->cfg.n_experts;
     cudaStream_t s = h->last_stream;
-    if (perm && T > 0) CU_TRY(h, launch_perm_readout(h, T, s));
+    if (perm && T > 0 && !h->picks_only) CU_TRY(h, launch_perm_readout(h, T, s));
     CU_TRY(h, cudaStreamSynchronize(s));
     int rc = check_dev_err(h);
     if (rc != OMOE_OK) return rc;
@@ -693,6 +723,20 @@ int omoe_get_routing(omoe_handle *h, int32_t *topk_idx, float *topk_w, int32_t *
         if (offsets) memset(offsets, 0, sizeof(int32_t) * (E + 1));
         return OMOE_OK;
     }
+    if (h->picks_only) {
+        if (!counts && !offsets && !perm) return OMOE_OK;
+        int32_t *idx = nullptr, cnt[kMaxExperts], off[kMaxExperts + 1] = {0};
+        rc = read_picks(h, &idx, cnt);
+        if (rc == OMOE_OK) {
+            for (int e = 0; e < E; e++) off[e + 1] = off[e] + cnt[e];
+            if (counts) memcpy(counts, cnt, sizeof(int32_t) * E);
+            if (offsets) memcpy(offsets, off, sizeof(int32_t) * (E + 1));
+            if (perm)
+                for (size_t f = 0; f < n; f++) perm[off[idx[f]]++] = (int32_t)f;
+        }
+        free(idx);
+        return rc;
+    }
     if (counts) CU_TRY(h, cudaMemcpy(counts, h->counts, sizeof(int32_t) * E, cudaMemcpyDeviceToHost));
     if (offsets) CU_TRY(h, cudaMemcpy(offsets, h->offsets, sizeof(int32_t) * (E + 1), cudaMemcpyDeviceToHost));
     if (perm && n) CU_TRY(h, cudaMemcpy(perm, h->perm_out, n * 4, cudaMemcpyDeviceToHost));
@@ -701,7 +745,6 @@ int omoe_get_routing(omoe_handle *h, int32_t *topk_idx, float *topk_w, int32_t *
 
 int omoe_get_logits(omoe_handle *h, float *logits) {
     if (!h || !logits) return OMOE_ERR_INVALID;
-    if (int rc = whole_batch_routing(h, h->last_stream)) return rc;
     CU_TRY(h, cudaStreamSynchronize(h->last_stream));
     const size_t n = (size_t)h->last_T * h->cfg.n_experts;
     if (n) CU_TRY(h, cudaMemcpy(logits, h->logits, n * 4, cudaMemcpyDeviceToHost));

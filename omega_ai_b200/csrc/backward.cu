@@ -776,7 +776,7 @@ int bw_set_aux(omoe_handle *h, float coef) {
     return OMOE_OK;
 }
 
-int bw_aux_loss(omoe_handle *h, float *loss_host, cudaStream_t s) {
+int bw_aux_loss(omoe_handle *h, float *loss_host, cudaStream_t s, const int32_t *counts_host) {
     BwState *b = static_cast<BwState *>(h->bw);
     if (!b) {
         snprintf(h->err, sizeof(h->err), "omoe_get_aux_loss: switch training mode on first");
@@ -790,13 +790,14 @@ int bw_aux_loss(omoe_handle *h, float *loss_host, cudaStream_t s) {
     int32_t cnt[kMaxExperts];
     if (cudaGetLastError() != cudaSuccess ||
         cudaMemcpyAsync(ps, b->aux_ps, sizeof(float) * E, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(cnt, h->counts, sizeof(int32_t) * E, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        (!counts_host && cudaMemcpyAsync(cnt, h->counts, sizeof(int32_t) * E, cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
         cudaStreamSynchronize(s) != cudaSuccess) {
         snprintf(h->err, sizeof(h->err), "omoe_get_aux_loss: CUDA error");
         return OMOE_ERR_CUDA;
     }
+    if (!counts_host) counts_host = cnt;
     float loss = 0.f;
-    for (int e = 0; e < E; e++) loss += ((float)cnt[e] / ((float)T * (float)k)) * (ps[e] / (float)T);
+    for (int e = 0; e < E; e++) loss += ((float)counts_host[e] / ((float)T * (float)k)) * (ps[e] / (float)T);
     *loss_host = (float)E * loss;
     return OMOE_OK;
 }

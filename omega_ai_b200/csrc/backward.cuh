@@ -20,7 +20,8 @@ int bw_backward_block(omoe_handle *h, const void *x, const float *gamma, float e
 int bw_get_grads(omoe_handle *h, float *d_router, float *d_bias, float *d_gate, float *d_up, float *d_down,
                  cudaStream_t s);
 int bw_set_aux(omoe_handle *h, float coef);
-int bw_aux_loss(omoe_handle *h, float *loss_host, cudaStream_t s);
+// counts_host: picks per expert, or null to take them from the device.
+int bw_aux_loss(omoe_handle *h, float *loss_host, cudaStream_t s, const int32_t *counts_host);
 void bw_destroy(omoe_handle *h);
 
 // 2-D bf16 tensor map: [rows, cols] with `ld` elements between rows, box box_rows x 64 columns, 128-byte swizzle.

@@ -122,10 +122,9 @@ struct omoe_handle {
     cudaEvent_t ev_in[omoe::kHostChunksMax], ev_out[omoe::kHostChunksMax], ev_set_fwd[2], ev_set_d2h[2];
     int host_chunk_min;     // smallest chunk (tokens) worth its own forward, one GPU
     int host_chunk_min_ep;  // the same with expert parallelism
-    // The last call was a host-buffer forward cut into chunks: its whole batch as staged (0 tokens: it was not).  The routing arrays
-    // hold the last chunk until a read-out asks for them (whole_batch_routing in api.cu).
-    const void *whole_x;
-    int whole_T, whole_io;
+    // The last_T rows that the read-outs describe ran in several forwards: logits, picks and gate weights are all there, the counts
+    // and positions only of the last forward's rows.
+    bool picks_only;
     bool host_pending;      // an omoe_forward_host_async call has not been waited for yet
 
     omoe::TensorMaps maps;
