@@ -95,7 +95,6 @@ def test_training_forward_is_followed_by_its_backward(T):
     layer.set_training(True)
     dy = torch.randn_like(last)
     layer.forward_host(xh, yh)
-    assert layer.launch_count() < cut
     read_logits(layer, T)
     layer.routing(T)
     dx = layer.backward(last, dy).clone()
