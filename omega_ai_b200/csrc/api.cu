@@ -280,6 +280,7 @@ int omoe_create(const omoe_config *cfg, omoe_handle **out) {
     if (const char *v = getenv("OMOE_HOST_CHUNK_MIN")) {
         h->host_chunk_min = atoi(v) > 0 ? atoi(v) : 1 << 30;
         h->host_chunk_min_ep = h->host_chunk_min;
+        h->host_chunk_min_set = true;
     }
     bool ok_streams = cudaStreamCreateWithFlags(&h->copy_in, cudaStreamNonBlocking) == cudaSuccess &&
                       cudaStreamCreateWithFlags(&h->copy_out, cudaStreamNonBlocking) == cudaSuccess;
@@ -568,19 +569,32 @@ static HostChunk host_chunk(int T, int pieces, int sub, int i) {
     return HostChunk{p.t0 + c.t0, c.n, p.t0};
 }
 
-// One GPU, batches below host_chunk_min per chunk: whether cutting into `chunks` still pays.  A chunk's copy has to
-// outlast the fixed part of one more forward (4 MB is about 75 us over PCIe against 45 us), its products have to stay bound by arithmetic and not by
-// reading the weights once more (512 rows per expert are twice the rows at which the two take the same time), and they have
-// to run on the same kernels as the whole batch's, so that every row keeps its bits.  Measured: 4096 tokens, d 1024, d_ff 2816, 8 experts
-// top-2 in one piece 478 us, in two 392 us.
+// One GPU, fewer than host_chunk_min tokens per chunk: whether pieces * sub chunks pay against half as many.  Every copy-in but the
+// first and every copy-out but the last runs beside kernels, so the call saves a chunk's copy both ways (56 GB/s over PCIe) and
+// pays for chunks / 2 more forwards: 80 us each and half of the time that the weights take from HBM (about 6 TB/s; the rest hides behind
+// arithmetic).  Measured for nine layers (d 512 to 4096, 35 MB to 2.8 GB of weights) at nine batches of 512 to 8184 rows: the 33 cuts
+// in two that this takes ran in 0.71 to 0.97 of the time of one piece (4096 rows, d 1024, d_ff 2816, 8 experts top-2: 489 -> 388 us), the
+// five in four in 0.80 to 0.94 of the time of two.  What it leaves out would have run in 0.89 to 1.4 in two and 0.84 to 1.9 in four, but for
+// layers so small that a chunk would run with K split.
 static bool chunk_pays(omoe_handle *h, int T, int pieces, int sub, size_t row_bytes) {
-    if (h->cfg.world != 1 || h->cfg.compute_dtype != OMOE_BF16 || h->host_chunk_min >= 1 << 30) return false;
-    // a backward follows a forward of the whole batch, and stage times are a forward's
-    if (bw_training(h) || h->profiling) return false;
-    const int chunks = pieces * sub;
-    const long rows = (long)(T / chunks) * h->cfg.top_k;
-    return (size_t)(T / chunks) * row_bytes >= (size_t)4 << 20 && rows >= 512l * h->cfg.n_experts &&
-           !experts_split_k(h, rows);
+    // a given minimum is the whole rule; a backward follows a forward of all its rows; stage times are a forward's
+    if (h->cfg.world != 1 || h->cfg.compute_dtype != OMOE_BF16 || h->host_chunk_min_set || bw_training(h) || h->profiling)
+        return false;
+    const int chunks = pieces * sub, least = host_chunk(T, pieces, sub, chunks - 1).n;  // the last chunk is the smallest
+    const double saved_ns = 2.0 * least * row_bytes / 56.0;
+    const double weights = 3.0 * 2.0 * h->cfg.n_experts * h->cfg.d_model * h->cfg.d_ff;
+    // and every chunk has to run on the kernels of the whole, so that every row keeps its bits
+    return least > 0 && saved_ns >= chunks / 2 * (80e3 + weights / 12e3) && !experts_split_k(h, (long)least * h->cfg.top_k);
+}
+
+// Page-locked memory: a copy to or from it does not hold the host up.
+static bool page_locked(const void *p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeHost;
 }
 
 // Enqueues one host-buffer forward: H2D copies, the forward(s), D2H copies.  No host synchronisation.
@@ -607,7 +621,10 @@ static int forward_host_enqueue(omoe_handle *h, const void *x_host, void *y_host
         const int basis = h->cfg.world == 1 ? T : h->cfg.t_max;
         const int cmin = h->cfg.world == 1 ? h->host_chunk_min : h->host_chunk_min_ep;
         while (pieces < kHostChunksMax && basis / (pieces * 2) >= cmin) pieces *= 2;
-        while (pieces * sub < kHostChunksMax && chunk_pays(h, T, pieces, sub * 2, row_bytes)) sub *= 2;
+        // with pageable buffers the host waits for each copy before it can launch the next chunk: nothing would overlap
+        while (pieces * sub < kHostChunksMax && chunk_pays(h, T, pieces, sub * 2, row_bytes) &&
+               (sub > 1 || (page_locked(x_host) && page_locked(y_host))))
+            sub *= 2;
     }
     const int chunks = pieces * sub;
     const int set = h->stage_next;

@@ -104,3 +104,20 @@ def test_training_forward_is_followed_by_its_backward(T):
     for name, g in layer.weight_grads().items():
         assert torch.equal(g, grads[name]), name
     layer.close()
+
+
+def test_pageable_buffers_and_a_given_minimum_are_not_cut(monkeypatch):
+    """Copies from pageable memory hold the host up, so nothing would overlap; OMOE_HOST_CHUNK_MIN is the whole rule when given."""
+    T, shape = 4096, (1024, 2816, 8, 2)
+    layer, _, xd, xh, yh = make(T, *shape)
+    y = layer.forward_device(xd).cpu()
+    in_one = layer.launch_count()
+    for x, out in ((xh.clone(), yh), (xh, torch.empty_like(y)), (xh.clone(), torch.empty_like(y))):
+        layer.forward_host(x, out)
+        assert layer.launch_count() == in_one and torch.equal(out, y)
+    layer.close()
+    monkeypatch.setenv("OMOE_HOST_CHUNK_MIN", "2049")
+    layer, _, xd, xh, yh = make(T, *shape)
+    layer.forward_host(xh, yh)
+    assert layer.launch_count() == in_one and torch.equal(yh, y)
+    layer.close()
