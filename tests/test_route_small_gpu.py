@@ -1,5 +1,5 @@
 """One-launch routing of a decode step (route_small.cu): rows that end inside a 256-column piece, rows longer than the
-shared-memory chunk, expert counts that are no multiple of a warp's."""
+shared-memory chunk, expert counts that are no multiple of a warp's, and both sides of the rule for a single block."""
 import pytest
 import torch
 
@@ -10,7 +10,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("io", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("T,d,E,k", [(1, 72, 1, 1), (8, 264, 128, 16), (3, 4096, 5, 2), (8, 4104, 33, 4), (5, 8200, 65, 3)])
+@pytest.mark.parametrize("T,d,E,k", [
+    (1, 72, 1, 1), (8, 264, 128, 16), (3, 4096, 5, 2), (8, 4104, 33, 4), (5, 8200, 65, 3),
+    (1, 3072, 8, 2), (1, 3080, 8, 2), (2, 1536, 8, 3), (1, 1544, 16, 4), (1, 2056, 5, 2), (1, 128, 17, 3),  # one block, or just not
+])
 def test_routing_of_a_few_tokens(oracle, T, d, E, k, io):
     dff = 64
     x, w_r, w_g, w_u, w_d, _ = make_layer(T, d, dff, E, k, seed=d + E)
