@@ -14,6 +14,8 @@ pytestmark = pytest.mark.gpu
     (1030, 264, 776, 2, 2),    # five equal token tiles per expert; tails in both feature counts
     (769, 1032, 136, 4, 2),    # one feature tile and a bit, K just past a multiple of 64
     (2100, 128, 2056, 24, 5),  # ragged experts
+    (300, 1032, 1032, 32, 4),  # no expert above 64 rows: nine narrow stages
+    (640, 1032, 1032, 32, 4),  # none above 128: eight
 ])
 def test_forward_at_tile_edges(oracle, T, d, dff, E, k):
     x, w_r, w_g, w_u, w_d, _ = make_layer(T, d, dff, E, k, seed=T)
@@ -25,7 +27,7 @@ def test_forward_at_tile_edges(oracle, T, d, dff, E, k):
     assert_close_bf16(y, r.y)
 
 
-@pytest.mark.parametrize("T", [1, 31, 32, 33, 64, 255, 256, 257, 481])
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 64, 65, 100, 128, 129, 255, 256, 257, 481])
 def test_training_step_at_tile_edges(oracle, T):
     """Both experts hold all T rows (top-2 of 2), so T is the width that the token tiles are cut from and the length the
     weight gradients reduce over."""
