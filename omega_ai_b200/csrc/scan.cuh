@@ -26,30 +26,30 @@ __device__ __forceinline__ void scan_body(const int32_t *__restrict__ block_coun
             // four blocks per lane and step (16-byte loads and stores) and the loads of eight steps together: the round
             // trips to L2 are all this kernel's time
             for (int b8 = 0; b8 < n_blocks; b8 += 8 * 128) {
-            int4 ahead[8];
+                int4 ahead[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int b = b8 + u * 128 + lane * 4;
-                ahead[u] = b < n_blocks ? *reinterpret_cast<const int4 *>(row + b) : make_int4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                if (b8 + u * 128 >= n_blocks) break;
-                const int b = b8 + u * 128 + lane * 4;
-                const int4 c4 = ahead[u];
-                const int sum4 = c4.x + c4.y + c4.z + c4.w;
-                int inc = sum4;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    int v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += v;
+                for (int u = 0; u < 8; u++) {
+                    const int b = b8 + u * 128 + lane * 4;
+                    ahead[u] = b < n_blocks ? *reinterpret_cast<const int4 *>(row + b) : make_int4(0, 0, 0, 0);
                 }
-                if (b < n_blocks) {
-                    const int base = run + inc - sum4;
-                    *reinterpret_cast<int4 *>(out + b) = make_int4(base, base + c4.x, base + c4.x + c4.y, base + c4.x + c4.y + c4.z);
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    if (b8 + u * 128 >= n_blocks) break;
+                    const int b = b8 + u * 128 + lane * 4;
+                    const int4 c4 = ahead[u];
+                    const int sum4 = c4.x + c4.y + c4.z + c4.w;
+                    int inc = sum4;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        int v = __shfl_up_sync(0xffffffffu, inc, o);
+                        if (lane >= o) inc += v;
+                    }
+                    if (b < n_blocks) {
+                        const int base = run + inc - sum4;
+                        *reinterpret_cast<int4 *>(out + b) = make_int4(base, base + c4.x, base + c4.x + c4.y, base + c4.x + c4.y + c4.z);
+                    }
+                    run += __shfl_sync(0xffffffffu, inc, 31);
                 }
-                run += __shfl_sync(0xffffffffu, inc, 31);
-            }
             }
             if (lane == 0) s_cnt[e] = run;
             continue;
