@@ -171,9 +171,9 @@ OMOE_API int omoe_wait(omoe_handle *h);
  * following omoe_forward / omoe_forward_block keep what the backward needs: the pre-activation rows of
  * the gate and up products, h, the expert outputs and the routing.  The reference's layers keep the same
  * things as the output tensors of linear1, the SiLU layer and linear3
- * (src/main/java/com/omega/engine/nn/layer/llama/LlamaMLPLayer.java:117-123).  A training-mode forward runs
- * the gate and up products unfused (their outputs must be stored) and rounds g and u to the compute dtype
- * before SiLU; on a bf16 layer its output can differ from the inference forward's in the last bf16 place.
+ * (src/main/java/com/omega/engine/nn/layer/llama/LlamaMLPLayer.java:117-123).  A training-mode forward stores
+ * the gate and up products' results, rounds them to the compute dtype before SiLU and takes that in full fp32
+ * accuracy; on a bf16 layer its output can differ from the inference forward's in the last bf16 place.
  * omoe_set_training(h, 0) goes back to the inference kernels and keeps the buffers.
  *
  * omoe_backward replaces LlamaMLPLayer.diff() (LlamaMLPLayer.java:139-158) and the FullyLayer.diff() calls

@@ -120,7 +120,7 @@ struct omoe_handle {
     // per chunk of a call: rows staged on the device / forward done; per staging set: the last call that used it
     // has consumed the staged rows / has copied its outputs back
     cudaEvent_t ev_in[omoe::kHostChunksMax], ev_out[omoe::kHostChunksMax], ev_set_fwd[2], ev_set_d2h[2];
-    int host_chunk_min;     // smallest chunk (tokens) worth its own forward, one GPU
+    int host_chunk_min;     // smallest chunk (tokens) that the interface states, one GPU; chunk_pays in api.cu cuts further
     int host_chunk_min_ep;  // the same with expert parallelism
     bool host_chunk_min_set;  // OMOE_HOST_CHUNK_MIN gave them: they are the whole rule
     // The last_T rows that the read-outs describe ran in several forwards: logits, picks and gate weights are all there, the counts

@@ -13,9 +13,9 @@
 // column operand may have any width that is a multiple of 32, so the tokens of an expert are cut into tiles of
 // equal width (<= 256) and the padding work of a 128-row token tile goes away with it.
 //
-// Measured against the kernel of experts_sm100.cu (128 x 256 tiles, one CTA each), whole layer: 16384 tokens, d 4096,
-// d_ff 14336, 8 experts top-2 10.27 -> 9.92 ms; 1531 tokens, d 1544, d_ff 4104, 12 experts top-3 355 -> 306 us; 4096
-// tokens on d 1024, d_ff 2816 the same within 1 %.  That kernel stays for expert
+// Measured against the kernel of experts_sm100.cu (128 x 256 tiles, one CTA each): 4096 tokens, d 1024, d_ff 2816, 8 experts top-2
+// up/gate 97 -> 73.5 us, down 45 -> 42.9; whole layer with 1531 tokens, d 1544, d_ff 4104, 12 experts top-3 358 -> 302 us; with 16384
+// tokens, d 4096, d_ff 14336, under the power cap 10.50 -> 9.90 ms where one side's runs differ by 2 to 6 %.  That kernel stays for expert
 // parallelism, whose rows it waits for and sends, and for a down product that it runs in one round (launch_experts_bf16).
 //
 // The accumulator comes out transposed (tensor-memory lane = output feature, column = token).  For up/gate the A tile
