@@ -55,8 +55,8 @@ CONFIGS = {
 SEED = 20240611
 X_BLOCK = 2048  # rows of x are drawn in blocks of this many tokens of the GLOBAL batch, one seed per block
 # dram__bytes_read.sum + dram__bytes_write.sum of one up/gate launch, from the ncu capture summarised in
-# profiles/grouped_gemm_ncu_full.md (full config-3 workload on one GPU); null for every other workload.
-NCU_TRAFFIC_BYTES = {("c3", 16384, 1): 5917402368 + 950249216}
+# profiles/pair_kernels_ncu.md (full config-3 workload on one GPU); null for every other workload.
+NCU_TRAFFIC_BYTES = {("c3", 16384, 1): 11580000000 + 943000000}
 
 
 def load_peaks():
@@ -759,8 +759,8 @@ def run_ours(args, cfg):
         dur = (stage_ms["up_gate"] + stage_ms["down"]) * 1e-3
         # which kernels ran depends on the step: the streaming kernels for one or two tokens, the split-K cluster
         # kernels while a product's tiles fit one round of resident clusters, else the persistent kernels
-        roof = {"bound": "hbm", "kernel": "expert products (up/gate + down): decode_gemv / grouped_gemm_splitk / "
-                                          "grouped_gemm kernels, picked per step",
+        roof = {"bound": "hbm", "kernel": "expert products (up/gate + down): decode_mma / grouped_gemm_splitk / "
+                                          "pair_gemm kernels, picked per step",
                 "achieved": wbytes / dur / 1e9, "peak": peaks["hbm"], "unit": "GB/s",
                 "frac": wbytes / dur / 1e9 / peaks["hbm"], "traffic": None, "peak_source": peaks["src"],
                 "active_experts": n_active, "weight_bytes": wbytes,
@@ -771,7 +771,8 @@ def run_ours(args, cfg):
         ach = alg["up_gate_flops"] / dur / 1e12
         timed_s = ms * 1e-3
         peak = peaks["tf_sust"] if timed_s >= 1.0 else peaks["tf_burst"]
-        roof = {"bound": "tensor", "kernel": "grouped_gemm_kernel<SWIGLU> (up/gate)", "achieved": ach,
+        roof = {"bound": "tensor", "achieved": ach,
+                "kernel": "pair_gemm_kernel (up/gate)" if world == 1 else "grouped_gemm_kernel<SWIGLU> (up/gate)",
                 "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                 "traffic": NCU_TRAFFIC_BYTES.get((args.config, T, world)),
                 "algorithmic_dram_bytes": 2.0 * (2 * El * d * dff + T_local * k * (d + dff)),

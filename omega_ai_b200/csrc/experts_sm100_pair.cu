@@ -45,10 +45,10 @@ constexpr int kStageBytesP = 2 * kABytesP;        // and up to 128 of the tile's
 // columns, kPass of them staged at a time.  Six stages and 2 x 16 KB of results fit; the epilogues that move three
 // results, or two rows in and two out, take a stage for their staging (five stages instead of six cost 1 % of a forward) and have
 // twice the warps: with eight, shared-memory words, exponentials and arithmetic of a pass follow one another and a tile's
-// epilogue outlasts a reduction of 1024.  Sixteen gain nothing for the other two.  Against a pass over the
-// accumulator per result and a SwiGLU kernel between the products: training step of
-// 4096 tokens, d 1024, d_ff 2816 673 -> 661 us, with the second eight warps 640 us; of 8192 tokens, d 4096, d_ff 14336
-// 18.3 -> 17.9 ms.
+// epilogue outlasts a reduction of 1024 (training step of 4096 tokens, d 1024, d_ff 2816 764 us, with sixteen 727).  Sixteen gain
+// nothing for the other two.
+// Both epilogues are bound by instructions there, a third of them the exponential and the divisions of full accuracy; with
+// __expf and __fdividef in their place the step takes 667 us, but the SiLU of a large negative g is off or zero (sm100_ptx.cuh).
 template <PairKind KIND>
 struct PairCfg {
     static constexpr bool kWide = KIND == PairKind::kUpGateKeep || KIND == PairKind::kSwigluBack;
