@@ -7,8 +7,8 @@
 // what counts is round trips to memory: every SM fetches one row, all of it at once, and every load of a thread is
 // requested before the first is used.  The block that finishes last picks the experts, turns the
 // picks into counts, offsets, row positions and the tile table, and copies the token rows into the dispatch buffer.
-// A step of one or two tokens on few experts and narrow rows runs in one block instead, whose warps take a (token, expert) pair each:
-// there is nothing to join then (launch_pl).
+// A step of one token on few experts and narrow rows runs in one block instead, a warp per expert: there is nothing to join then
+// (launch_pl).
 // Measured against a block per token whose warps walked the experts (loads inside a bounds branch, each waited for before
 // the next): step of 8 tokens, d 2048, 64 experts 144.5 -> 124 us (this kernel 33 -> 14 us), of one token, d 4096, 8 experts
 // 132 -> 126 us.
@@ -65,11 +65,9 @@ route_small_kernel(const XT *__restrict__ x, const float *__restrict__ w_r, cons
     pdl_trigger();
     pdl_wait();  // the step before may still be reading the routing arrays this kernel overwrites
 
-    const bool alone = gridDim.x == 1;  // one block does it all: a warp per (token, expert), nothing to join
+    const bool alone = gridDim.x == 1 && T == 1;  // one block does it all: a warp per expert, nothing to join
     if (alone) {
-        for (int p = warp; p < T * E; p += 8) {
-            const int t = p / E, e = p - t * E;
-            const XT *xr = x + (size_t)t * d;
+        for (int e = warp; e < E; e += 8) {
             const float *wr = w_r + (size_t)e * d;
             float even = 0.f, odd = 0.f;
             for (int i0 = lane * 8; i0 < d; i0 += kAhead * 256) {
@@ -77,7 +75,7 @@ route_small_kernel(const XT *__restrict__ x, const float *__restrict__ w_r, cons
                 Raw8<float> wv[kAhead];
 #pragma unroll
                 for (int u = 0; u < kAhead; u++) {  // addresses past the row are clamped, not branched around
-                    xv[u].load(xr + min(i0 + u * 256, d - 8));
+                    xv[u].load(x + min(i0 + u * 256, d - 8));
                     wv[u].load(wr + min(i0 + u * 256, d - 8));
                 }
 #pragma unroll
@@ -98,7 +96,7 @@ route_small_kernel(const XT *__restrict__ x, const float *__restrict__ w_r, cons
             for (int m = 16; m >= 1; m >>= 1) v = v + __shfl_xor_sync(0xffffffffu, v, m);
             if (lane == 0) {
                 if (bias != nullptr) v = v + __ldg(bias + e);
-                sl[t][e] = logits[p] = v;
+                sl[0][e] = logits[e] = v;
             }
         }
         __syncthreads();
@@ -239,13 +237,12 @@ route_small_kernel(const XT *__restrict__ x, const float *__restrict__ w_r, cons
 
 template <int PL, typename XT>
 cudaError_t launch_pl(omoe_handle *h, const XT *x, int T, cudaStream_t s) {
-    const int E = h->cfg.n_experts, per_warp = (T * E + 7) / 8;
-    // One block where its warps have one or two products each and at most 3072 columns of them, about one round trip's loads:
-    // joining the blocks (fence, ticket, logits back from L2) costs more than a narrow row's loads.  Whole step of one token with
-    // one block and with a block per expert, 8 experts: d 256 12.4 us against 14.2; d 1024 15.3 against 16.8; d 2048 18.9
-    // against 20.9; d 3072 25.0 against 25.5; 16 experts of d 2048 21.4 against 21.2; 32 of d 512 (four products a warp) 19.3 against
-    // 18.8; two tokens, 8 experts, d 2048 32.7 against 31.3.
-    const bool alone = per_warp <= 2 && per_warp * h->cfg.d_model <= 3072;
+    const int E = h->cfg.n_experts, per_warp = (E + 7) / 8;
+    // One block for one token where its warps' products are at most 1536 columns together, a round trip's loads: joining the blocks
+    // (fence, ticket, logits back from L2) costs more than a narrow row's loads. Whole step with one block and with a block per expert, all
+    // rows cold: 8 experts top-1 d 512 17.4 us against 19.1, top-2 d 1024 28.0 against 30.4, d 1536 28.2 against 29.5, but d 2040 45.3 against
+    // 43.9; 16 experts d 512 24.4 against 25.3, but d 1536 33.1 against 30.3.  Two tokens, 8 experts, d 1024: 44 against 38.
+    const bool alone = T == 1 && per_warp * h->cfg.d_model <= 1536;
     return launch_ex(route_small_kernel<PL, XT>, dim3(alone ? 1 : E), dim3(256), 0, s, h->pdl, x, h->w_router, h->router_bias, T,
                      h->cfg.d_model, E, h->cfg.top_k, h->cfg.renormalize, h->logits, h->topk_idx, h->topk_w, h->counts,
                      h->offsets, h->poffsets, h->tile_expert, (int)(h->rows_cap / kRowAlign), h->pos,

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("io", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T,d,E,k", [
     (1, 72, 1, 1), (8, 264, 128, 16), (3, 4096, 5, 2), (8, 4104, 33, 4), (5, 8200, 65, 3),
-    (1, 3072, 8, 2), (1, 3080, 8, 2), (2, 1536, 8, 3), (1, 1544, 16, 4), (1, 2056, 5, 2), (1, 128, 17, 3),  # one block, or just not
+    (1, 1536, 8, 2), (1, 1544, 8, 2), (2, 1536, 8, 3), (1, 768, 16, 4), (1, 776, 16, 4), (1, 1000, 5, 2), (1, 128, 17, 3),  # one block, or just not
 ])
 def test_routing_of_a_few_tokens(oracle, T, d, E, k, io):
     dff = 64
